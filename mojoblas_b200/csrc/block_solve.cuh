@@ -1,5 +1,4 @@
-// Fused diagonal-block triangular solve, shared by the blocked trsm (trsm.cu)
-// and the grouped strsm plans (grouped.cu).  Included by both translation units.
+// Fused diagonal-block triangular solve of the blocked trsm (trsm.cu).
 #pragma once
 
 #include "mbg_internal.cuh"
@@ -18,10 +17,10 @@ constexpr int BS_THREADS = 8 * BS_COLS;           // eight lanes per column in t
 constexpr int BS_TILE = NB * 72;                  // diagonal block + reciprocals (64 x 65 + 64), or a 64 x 72 tile
 
 inline int bs_strip_ld(int nb) { return (int)(cdiv(nb, NB) * NB) + 2; }
-// nbuf: staging buffers per strip (items staged nbuf - 1 ahead of the one being computed)
+constexpr int NBUF = 2;  // staging buffers per strip (items staged NBUF - 1 ahead of the one being computed)
 template <typename T>
-inline size_t bs_smem_bytes(int nb, int nbuf = 2) {
-    return sizeof(T) * (size_t(BS_COLS) * bs_strip_ld(nb) + size_t(nbuf) * BS_TILE);
+inline size_t bs_smem_bytes(int nb) {
+    return sizeof(T) * (size_t(BS_COLS) * bs_strip_ld(nb) + size_t(NBUF) * BS_TILE);
 }
 
 // One element copied global -> shared without a register round trip; zero-filled
@@ -58,14 +57,13 @@ __device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.w
 // The diagonal blocks and tiles form one sequence per strip that is staged
 // with cp.async into NBUF rotating buffers: the next NBUF - 1 items are in flight
 // while the current one is computed, so the L2 latency of A (shared by every
-// CTA) is hidden.  Two for the blocked trsm (a third measured slower there); three
-// for the grouped plans' small problems (measured 9 % faster).  The strip is read from and written to HBM once; only
+// CTA) is hidden (a third buffer measured slower).  The strip is read from and written to HBM once; only
 // off-diagonal blocks above the launch's size go through gemm.  Rows at or
 // past nb stay zero in the strip and staged items are zero outside op(A)'s
 // block, so ragged edges need no special case in the inner loops.
 // IDENT: the right-hand side is the identity (columns c0 .. of the nb x nb block inverse),
 // generated in shared memory instead of read from B; B is only written.
-template <typename T, bool LOWER, bool TRANS, bool UNIT, int W, int NBUF = 2, bool IDENT = false>
+template <typename T, bool LOWER, bool TRANS, bool UNIT, int W, bool IDENT = false>
 __device__ __forceinline__ void block_solve_strip(int nb, i64 ncols, const T* __restrict__ A, i64 lda,
                                                   T* __restrict__ B, i64 ldb, i64 c0, T alpha,
                                                   unsigned char* bs_smem_raw) {
@@ -76,7 +74,6 @@ __device__ __forceinline__ void block_solve_strip(int nb, i64 ncols, const T* __
     constexpr int LT = TRANS ? NB + 2 : NB + 8;  // update tile: [l][r] (plain) or [r][l] (transposed)
     const int nsub = (nb + NB - 1) / NB, nbr = nsub * NB, ldbs = nbr + 2;
     T* Bs = reinterpret_cast<T*>(bs_smem_raw);
-    static_assert(NBUF >= 2, "staging depth");
     T* const buf0 = Bs + (size_t)W * ldbs;  // NBUF staging buffers of BS_TILE elements
     const int tid = threadIdx.x;
 

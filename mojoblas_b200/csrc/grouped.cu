@@ -4,7 +4,7 @@
 // The reference has no batched interface; a mojoBLAS caller loops over its
 // gemm (src/level3/gemm.mojo:56) / trsm (src/level3/trsm.mojo:20) calls.  Here
 // a host-side plan uploads a problem table once, and each execution is a CUDA
-// graph of [reset the tile counter; one persistent kernel]:
+// graph of its kernels (a tile counter's reset before each persistent one):
 //
 //  * sgemm: problems are ordered by k * m * n descending and cut into square
 //    tiles (64 or 128, from the tuning table); persistent CTAs take tiles from
@@ -13,16 +13,13 @@
 //    tile code of gemm_f32_tile.cuh with that problem's transposes, alpha and
 //    beta (16-byte copies where that problem's operands allow them).
 //  * strsm (left side, any uplo / trans / diag, n <= 256): problems are cut
-//    into strips of 32 right-hand sides, ordered largest problem first;
-//    persistent CTAs take strips from an atomic counter and solve each with
-//    the blocked trsm's fused diagonal-block routine (block_solve.cuh): the
-//    strip in shared memory, the reference's column substitution
-//    (src/level3/trsm.mojo:111-168) on 64-row sub-blocks with the pivot
-//    broadcast by a shuffle and multiplied by a precomputed reciprocal, and the
-//    updates between sub-blocks from cp.async-staged tiles of op(A).
+//    into strips of 32 right-hand sides, each solved by one or two warps
+//    (warp_solve.cuh: rows of one right-hand side in one thread's registers, the
+//    reference's column substitution, src/level3/trsm.mojo:111-168, on 32-row blocks);
+//    the plan packs the strips into CTAs of four warps, largest problems first.
 #include "mbg_internal.cuh"
-#include "block_solve.cuh"
 #include "gemm_f32_tile.cuh"
+#include "warp_solve.cuh"
 
 #include <algorithm>
 #include <numeric>
@@ -106,49 +103,84 @@ struct TrsmDesc {
 };
 
 constexpr int TR_MAXN = 256;  // largest problem order a grouped strsm plan takes
-constexpr int GS_NBUF = 3;    // staging buffers per strip of the fused block solve
+constexpr int GS_WARPS = 4;    // warps per CTA
+constexpr int GS_MAXBLK = TR_MAXN / ws::RB;
+constexpr int GS_SLOTS = GS_MAXBLK + 2 * GS_WARPS;  // shared memory per CTA in 4 KB slots: a strip of the largest order
+constexpr int GS_SMEM = GS_SLOTS * ws::SLOT * int(sizeof(float));
 
-// One unit of grouped-strsm work: a strip of up to bs::BS_COLS right-hand sides of one problem.
-struct TrsmItem {
-    int prob;
-    int pad_;
-    i64 c0;
+// Warps of a strip of nblk row blocks: what covers the chain of its diagonal blocks without
+// leaving warps idle.  Measured on the 2048 problems below: at most two warps from five
+// blocks on 0.092 ms, from three on 0.090; four from five on 0.081, and two from three on
+// 0.077; four from three on 0.081.
+inline int gs_strip_warps(int nblk) { return nblk >= 5 ? 4 : nblk >= 3 ? 2 : 1; }
+
+// One warp's work: part wi of W of a strip of up to 32 right-hand sides of one problem.
+struct TrsmSlot {
+    int prob;   // -1: nothing
+    int wi, W;
+    int x, ring, bar;  // the strip's first X slot, the warp's ring, the strip's first mbarrier
+    i64 c0;     // first right-hand side
 };
 
-// Persistent grouped strsm: each CTA takes (problem, strip) items from an atomic
-// counter — the plan orders them largest problem first, so the long solves start
-// early and the small ones fill in behind them — and solves each with the fused
-// diagonal-block routine of the blocked trsm: the strip in shared memory, 64-row
-// substitution sub-blocks, cp.async-staged tiles of op(A), alpha applied to the
-// strip as it lands.
-__global__ void __launch_bounds__(bs::BS_THREADS, 2)
-grouped_block_strsm_kernel(const TrsmDesc* __restrict__ probs, const TrsmItem* __restrict__ items, int nitems,
-                           unsigned long long* __restrict__ counter) {
-    extern __shared__ __align__(16) unsigned char gs_smem[];
-    __shared__ int s_item;
-    for (;;) {
-        if (threadIdx.x == 0) s_item = int(atomicAdd(counter, 1ULL));
-        __syncthreads();
-        const int it = s_item;
-        __syncthreads();  // every thread has read s_item before thread 0 writes the next one
-        if (it >= nitems) break;
-        const TrsmItem w = items[it];
-        const TrsmDesc d = probs[w.prob];
-        const int nb = int(d.n);
-#define GS(L, TR, U)                                                                                  \
-    bs::block_solve_strip<float, L, TR, U, bs::BS_COLS, GS_NBUF>(nb, d.nrhs, d.a, d.lda, d.b, d.ldb, w.c0, d.alpha, gs_smem)
-        switch ((d.lower ? 4 : 0) | (d.trans ? 2 : 0) | (d.unit ? 1 : 0)) {
-            case 0: GS(false, false, false); break;
-            case 1: GS(false, false, true); break;
-            case 2: GS(false, true, false); break;
-            case 3: GS(false, true, true); break;
-            case 4: GS(true, false, false); break;
-            case 5: GS(true, false, true); break;
-            case 6: GS(true, true, false); break;
-            default: GS(true, true, true); break;
+// Grouped strsm: CTA i runs the slots of table row i, one per warp.  The plan packs strips
+// into CTAs by their warps and shared memory (warp_solve.cuh: a slot per row block of X and two
+// per warp), the largest problems first.  64 KB and 128 threads: three CTAs per SM (six or
+// eight warps to a CTA of 72 KB, which mixes long and short strips: 0.104 and 0.118 ms).
+// 2048 problems (order 8..256 log-uniform, 1..64 right-hand sides): 0.077 ms with the copy of
+// B, against 0.212 ms for persistent CTAs of eight lanes per column over 64-row sub-blocks.
+__global__ void __launch_bounds__(32 * GS_WARPS, 3)
+grouped_strsm_kernel(const TrsmDesc* __restrict__ probs, const TrsmSlot* __restrict__ slots, int* err) {
+    extern __shared__ __align__(16) float gs_smem[];
+    __shared__ uint64_t bars[2 * GS_MAXBLK];
+    __shared__ int zeros[GS_WARPS * GS_MAXBLK];  // a strip uses its first warp's
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const TrsmSlot s = slots[i64(blockIdx.x) * GS_WARPS + warp];
+    if (threadIdx.x < 2 * GS_MAXBLK) tc::mbar_init(&bars[threadIdx.x], 1);
+    __syncthreads();
+    if (s.prob < 0) return;
+    const TrsmDesc d = probs[s.prob];
+    const int n = int(d.n);
+    ws::Problem p;
+    ws::solve_order(p, d.a, d.lda, n, d.lower, d.trans);
+    p.b = d.b + s.c0 * d.ldb + (d.lower ? 0 : n - 1);
+    p.sb = d.lower ? 1 : -1;
+    p.ldb = d.ldb;
+    p.cols = int(min(i64(ws::RB), d.nrhs - s.c0));
+    p.alpha = d.alpha;
+    p.unit = d.unit;
+    ws::solve_strip<false>(p, s.wi, s.W, gs_smem + s.x * ws::SLOT, gs_smem + s.ring * ws::SLOT, bars + s.bar,
+                           zeros + (warp - s.wi) * GS_MAXBLK, lane, err);
+}
+
+// Packs the strips into CTAs: largest first, each into one of the last few CTAs with room.
+std::vector<TrsmSlot> pack_strips(const std::vector<TrsmDesc>& v) {
+    struct Strip { int prob, nblk; i64 c0; };
+    std::vector<Strip> strips;
+    for (int i = 0; i < int(v.size()); ++i)
+        for (i64 c0 = 0; c0 < v[size_t(i)].nrhs; c0 += ws::RB)
+            strips.push_back(Strip{i, int(cdiv(v[size_t(i)].n, ws::RB)), c0});
+    std::stable_sort(strips.begin(), strips.end(),
+                     [&](const Strip& x, const Strip& y) { return v[size_t(x.prob)].n > v[size_t(y.prob)].n; });
+    struct Cta { int warps = 0, slots = 0, bars = 0; };
+    std::vector<Cta> ctas;
+    std::vector<TrsmSlot> table;
+    constexpr size_t LOOK_BACK = 16;
+    for (const Strip& s : strips) {
+        const int W = gs_strip_warps(s.nblk), need = s.nblk + 2 * W;
+        size_t c = ctas.size() > LOOK_BACK ? ctas.size() - LOOK_BACK : 0;
+        while (c < ctas.size() && (ctas[c].warps + W > GS_WARPS || ctas[c].slots + need > GS_SLOTS)) ++c;
+        if (c == ctas.size()) {
+            ctas.push_back(Cta());
+            table.resize(table.size() + GS_WARPS, TrsmSlot{-1, 0, 0, 0, 0, 0, 0});
         }
-#undef GS
+        Cta& t = ctas[c];
+        for (int wi = 0; wi < W; ++wi)
+            table[c * GS_WARPS + size_t(t.warps++)] =
+                TrsmSlot{s.prob, wi, W, t.slots, t.slots + s.nblk + 2 * wi, W > 1 ? t.bars : 0, s.c0};
+        t.slots += need;
+        if (W > 1) t.bars += GS_MAXBLK;  // at most two strips of two warps
     }
+    return table;
 }
 
 // SMs of the current device (queried per plan: plans are built once, off the hot path)
@@ -184,9 +216,8 @@ struct mbg_plan {
     // sgemm, split forms (BF16x3 / BF16x6): the tensor-core grouped kernel
     bool tc = false;
     mbg::GroupedTcPlan tcp;
-    void* items = nullptr;  // strsm: (problem, strip) work items, inside the table allocation
-    int nitems = 0;
-    size_t smem = 0;        // strsm: dynamic shared memory per CTA
+    void* items = nullptr;  // strsm: the warps' work, a slot per warp, inside the table allocation
+    int* err = nullptr;     // strsm: the device's wait-error flag
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     cudaStream_t stream = nullptr;  // stream the graph was captured on
@@ -215,9 +246,8 @@ int enqueue_plan(mbg_plan* p, cudaStream_t s) {
         }
         return MBG_OK;
     }
-    MBG_CUDA(cudaMemsetAsync(p->counter, 0, sizeof(unsigned long long), s));
-    grouped_block_strsm_kernel<<<p->grid, bs::BS_THREADS, p->smem, s>>>(
-        static_cast<const TrsmDesc*>(p->table), static_cast<const TrsmItem*>(p->items), p->nitems, p->counter);
+    grouped_strsm_kernel<<<p->grid, 32 * GS_WARPS, GS_SMEM, s>>>(static_cast<const TrsmDesc*>(p->table),
+                                                                 static_cast<const TrsmSlot*>(p->items), p->err);
     return check_launch("grouped_strsm");
 }
 
@@ -407,44 +437,27 @@ int mbg_strsm_grouped_plan(int mode, int count, const mbg_strsm_problem* probs, 
         cols += q.n;
         v.push_back(d);
     }
-    // work items: 32-column strips, largest problem first (ties keep the caller's order)
-    std::vector<TrsmItem> items;
-    for (int i = 0; i < int(v.size()); ++i)
-        for (i64 c0 = 0; c0 < v[size_t(i)].nrhs; c0 += bs::BS_COLS) items.push_back(TrsmItem{i, 0, c0});
-    std::stable_sort(items.begin(), items.end(),
-                     [&](const TrsmItem& x, const TrsmItem& y) { return v[size_t(x.prob)].n > v[size_t(y.prob)].n; });
+    const std::vector<TrsmSlot> slots = pack_strips(v);
     mbg_plan* p = new mbg_plan();
     p->kind = 2;
     p->count = int(v.size());
     p->total = cols;
-    p->nitems = int(items.size());
-    p->smem = bs::bs_smem_bytes<float>(TR_MAXN, GS_NBUF);
     int st = MBG_OK;
     if (p->count > 0) {
-        int per_sm = 0;
-        cudaError_t e = cudaFuncSetAttribute(grouped_block_strsm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             int(p->smem));
-        if (e == cudaSuccess)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grouped_block_strsm_kernel, bs::BS_THREADS,
-                                                              p->smem);
+        p->grid = int(slots.size() / GS_WARPS);
+        p->err = device_error_flag();  // created here: its first use must not fall inside the graph capture
+        const size_t dbytes = (sizeof(TrsmDesc) * v.size() + 255) / 256 * 256;
+        const size_t sbytes = sizeof(TrsmSlot) * slots.size();
+        cudaError_t e = cudaFuncSetAttribute(grouped_strsm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GS_SMEM);
+        if (e == cudaSuccess) e = cudaMalloc(&p->table, dbytes + sbytes);
+        if (e == cudaSuccess) {
+            p->items = static_cast<char*>(p->table) + dbytes;
+            e = cudaMemcpy(p->table, v.data(), sizeof(TrsmDesc) * v.size(), cudaMemcpyHostToDevice);
+        }
+        if (e == cudaSuccess) e = cudaMemcpy(p->items, slots.data(), sbytes, cudaMemcpyHostToDevice);
         if (e != cudaSuccess) {
-            set_error("grouped strsm kernel set-up", e);
+            set_error("grouped strsm plan set-up", e);
             st = MBG_ERR_CUDA;
-        } else {
-            p->grid = int(imax(1, imin(i64(items.size()), i64(num_sms()) * imax(per_sm, 1))));
-            const size_t dbytes = (sizeof(TrsmDesc) * v.size() + 255) / 256 * 256;
-            const size_t ibytes = sizeof(TrsmItem) * items.size();
-            e = cudaMalloc(&p->table, dbytes + ibytes);
-            if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&p->counter), sizeof(unsigned long long));
-            if (e == cudaSuccess) {
-                p->items = static_cast<char*>(p->table) + dbytes;
-                e = cudaMemcpy(p->table, v.data(), sizeof(TrsmDesc) * v.size(), cudaMemcpyHostToDevice);
-            }
-            if (e == cudaSuccess) e = cudaMemcpy(p->items, items.data(), ibytes, cudaMemcpyHostToDevice);
-            if (e != cudaSuccess) {
-                set_error("grouped strsm plan upload", e);
-                st = MBG_ERR_CUDA;
-            }
         }
         if (!st) st = capture_plan(p);
     }

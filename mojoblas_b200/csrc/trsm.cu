@@ -29,6 +29,7 @@
 // triangle is nonzero.
 #include "mbg_internal.cuh"
 #include "block_solve.cuh"
+#include "warp_solve.cuh"
 
 #include <vector>
 
@@ -408,8 +409,49 @@ block_invert_kernel(i64 m, int nbi, const T* __restrict__ A, i64 lda, T* __restr
     const int nbb = int(min(i64(nbi), m - r0));
     const i64 c0 = i64(blockIdx.x) * BS_COLS;
     if (c0 >= nbb) return;
-    bs::block_solve_strip<T, LOWER, TRANS, UNIT, BS_COLS, 2, true>(nbb, nbb, A + r0 + r0 * lda, lda, W + r0, ldw, c0,
+    bs::block_solve_strip<T, LOWER, TRANS, UNIT, BS_COLS, true>(nbb, nbb, A + r0 + r0 * lda, lda, W + r0, ldw, c0,
                                                                    T(1), bs_smem_raw);
+}
+
+// The same for FP32 by the strip solve of warp_solve.cuh: strip j of a block's inverse is
+// zero above row 32 j, so it solves only the trailing rows.  Eight warps per strip: the first
+// strip's 120 tiles are bound by shared-memory reads, its diagonal blocks by their chain
+// (four blocks of 512 rows: 0.060 ms, 0.125 with block_solve_strip; 4 / 8 / 12 / 16
+// warps for the strsm adjoint of order 2048 with 512 right-hand sides: 0.280 / 0.270 /
+// 0.292 / 0.295 ms, 0.336 before).
+constexpr int INV_WARPS = 8;
+constexpr int INV_MAXBLK = 512 / ws::RB;  // blocks of up to 512 rows
+constexpr int INV_SMEM = (INV_MAXBLK + 2 * INV_WARPS) * ws::SLOT * int(sizeof(float));
+__global__ void __launch_bounds__(32 * INV_WARPS, 1)
+block_invert_f32_kernel(i64 m, int nbi, const float* __restrict__ A, i64 lda, bool lower, bool trans, bool unit,
+                        float* __restrict__ W, i64 ldw, int* err) {
+    extern __shared__ __align__(16) float inv_smem[];
+    __shared__ uint64_t bars[INV_MAXBLK];
+    const i64 r0 = i64(blockIdx.y) * nbi;
+    const int nbb = int(min(i64(nbi), m - r0)), c0 = int(blockIdx.x) * ws::RB;
+    if (c0 >= nbb) return;
+    if (threadIdx.x < INV_MAXBLK) tc::mbar_init(&bars[threadIdx.x], 1);
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // the block in solve order: an upper one reversed along both dimensions
+    const i64 dir = lower ? 1 : -1;
+    float* const w00 = W + r0 + (lower ? 0 : (nbb - 1) * (ldw + 1));
+    ws::Problem p;
+    ws::solve_order(p, A + r0 * (lda + 1), lda, nbb, lower, trans);
+    p.a += c0 * (p.sr + p.sl);
+    p.n = nbb - c0;
+    p.b = w00 + c0 * dir * (ldw + 1);
+    p.sb = dir;
+    p.ldb = dir * ldw;
+    p.cols = min(ws::RB, p.n);
+    p.alpha = 1.0f;
+    p.unit = unit;
+    for (int r = 32 * warp; r < c0; r += 32 * INV_WARPS) {
+        float* q = w00 + dir * (r + lane) + dir * c0 * ldw;
+        for (int c = 0; c < p.cols; ++c, q += dir * ldw) *q = 0.0f;
+    }
+    ws::solve_strip<true>(p, warp, INV_WARPS, inv_smem, inv_smem + (INV_MAXBLK + 2 * warp) * ws::SLOT, bars, nullptr, lane,
+                          err);
 }
 
 template <typename T>
@@ -433,6 +475,22 @@ int launch_block_invert_t(i64 m, int nbi, const T* a, i64 lda, T* w, i64 ldw) {
     return check_launch("trsm_block_invert");
 }
 
+int launch_block_invert_f32(bool lower, bool trans, bool unit, i64 m, int nbi, const float* a, i64 lda, float* w,
+                            i64 ldw) {
+    static std::atomic<unsigned> configured{0};  // one bit per device
+    int dev = 0;
+    MBG_CUDA(cudaGetDevice(&dev));
+    if (!configured_on(configured, dev)) {
+        MBG_CUDA(cudaFuncSetAttribute(block_invert_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      INV_SMEM));
+        mark_configured(configured, dev);
+    }
+    const dim3 g(unsigned(cdiv(nbi, ws::RB)), unsigned(cdiv(m, nbi)));
+    block_invert_f32_kernel<<<g, 32 * INV_WARPS, INV_SMEM, stream()>>>(m, nbi, a, lda, lower, trans, unit, w, ldw,
+                                                                       device_error_flag());
+    return check_launch("trsm_block_invert");
+}
+
 // W := the inverses of op(A)'s diagonal blocks of nbi rows, stacked (m x nbi, ld m).
 template <typename T>
 int invert_diagonal_blocks(bool lower, bool trans, bool unit, i64 m, int nbi, const T* a, i64 lda, T* w) {
@@ -444,15 +502,19 @@ int invert_diagonal_blocks(bool lower, bool trans, bool unit, i64 m, int nbi, co
     if (nb_last < nbi)
         MBG_CUDA(cudaMemset2DAsync(w + r_last + nb_last * m, size_t(m) * sizeof(T), 0, size_t(nb_last) * sizeof(T),
                                    size_t(nbi - nb_last), stream()));
-#define BIV(L, TR, U) return launch_block_invert_t<T, L, TR, U>(m, nbi, a, lda, w, m)
-    if (lower) {
-        if (trans) { if (unit) BIV(true, true, true); else BIV(true, true, false); }
-        else { if (unit) BIV(true, false, true); else BIV(true, false, false); }
+    if constexpr (sizeof(T) == 4) {
+        return launch_block_invert_f32(lower, trans, unit, m, nbi, a, lda, w, m);
     } else {
-        if (trans) { if (unit) BIV(false, true, true); else BIV(false, true, false); }
-        else { if (unit) BIV(false, false, true); else BIV(false, false, false); }
-    }
+#define BIV(L, TR, U) return launch_block_invert_t<T, L, TR, U>(m, nbi, a, lda, w, m)
+        if (lower) {
+            if (trans) { if (unit) BIV(true, true, true); else BIV(true, true, false); }
+            else { if (unit) BIV(true, false, true); else BIV(true, false, false); }
+        } else {
+            if (trans) { if (unit) BIV(false, true, true); else BIV(false, true, false); }
+            else { if (unit) BIV(false, false, true); else BIV(false, false, false); }
+        }
 #undef BIV
+    }
 }
 
 // The inverses' planes (bf16 split terms or Ozaki slices), made once per solve.

@@ -123,20 +123,72 @@ struct Params {
     int* err;
 };
 
+// Predicated accesses: a branch around each element's store took about 150 cycles a column
+// (a 128 x 256 tile stored in 20000 cycles, 10 us, against 94000 for a reduction of 2047).
+__device__ __forceinline__ void st_if(float* p, float v, int on) {
+    asm volatile("{ .reg .pred q; setp.ne.s32 q, %2, 0; @q st.global.f32 [%0], %1; }" ::"l"(p), "f"(v), "r"(on) : "memory");
+}
+__device__ __forceinline__ void add_if(float* p, float v, int on) {
+    asm volatile("{ .reg .pred q; setp.ne.s32 q, %2, 0; @q red.global.add.f32 [%0], %1; }" ::"l"(p), "f"(v), "r"(on)
+                 : "memory");
+}
+__device__ __forceinline__ float ld_if(const float* p, int on) {  // 0 where off
+    float v;
+    asm volatile("{ .reg .pred q; setp.ne.s32 q, %2, 0; mov.f32 %0, 0f00000000; @q ld.global.f32 %0, [%1]; }"
+                 : "=f"(v)
+                 : "l"(p), "r"(on)
+                 : "memory");
+    return v;
+}
+
+// The columns of a row that a product writes, as offsets [lo, hi) from column `col`: those below
+// `end`, in the triangle's mask; none for a row past the last.
+__device__ __forceinline__ void live_columns(const Params& P, const i64 row, const i64 col, const i64 end, int& lo,
+                                             int& hi) {
+    lo = 0;
+    hi = int(max(i64(0), end - col));
+    if (P.tri == 1) hi = int(max(i64(0), min(i64(hi), row - col + 1)));
+    if (P.tri == 2) lo = int(max(i64(0), min(i64(hi), row - col)));
+    if (row >= P.m) hi = lo;
+}
+
+// W columns of a row of C from p: alpha v (+ beta C) in columns [lo, hi).  beta == 1 (the trsm
+// updates) adds in L2, one add per element, rounded as c + v, with no read in the thread.
+template <int W>
+__device__ __forceinline__ void split_store(float* p, const i64 ldc, const float alpha, const float beta,
+                                            const float (&v)[W], const int lo, const int hi) {
+    const unsigned len = unsigned(hi - lo);
+    if (beta == 0.0f) {
+#pragma unroll
+        for (int j = 0; j < W; ++j, p += ldc) st_if(p, alpha * v[j], unsigned(j - lo) < len);
+    } else if (beta == 1.0f) {
+#pragma unroll
+        for (int j = 0; j < W; ++j, p += ldc) add_if(p, alpha * v[j], unsigned(j - lo) < len);
+    } else {
+#pragma unroll
+        for (int c0 = 0; c0 < W; c0 += 16) {  // sixteen loads of C in flight
+            float cv[16];
+            float* q = p;
+#pragma unroll
+            for (int j = 0; j < 16; ++j, q += ldc) cv[j] = ld_if(q, unsigned(c0 + j - lo) < len);
+#pragma unroll
+            for (int j = 0; j < 16; ++j, p += ldc)
+                st_if(p, fmaf(beta, cv[j], alpha * v[c0 + j]), unsigned(c0 + j - lo) < len);
+        }
+    }
+}
+
 // One output row's EPI_COLS columns from cbase of a split product: C = alpha acc (+ beta C),
 // the trmm form alpha acc + d .* C, triangle masks; columns past n are skipped.
 template <class C>
 __device__ __forceinline__ void split_store_row(const Params& P, const i64 row, const i64 cbase,
                                                 const float (&acc)[C::EPI_COLS]) {
     float* Cm = static_cast<float*>(P.c);
-    const float alpha = float(P.alpha), beta = float(P.beta);
-    // 8 columns at a time: all loads of C are issued before the
-    // first is used, so the read-modify-write of a beta != 0 call
-    // waits for memory once per 8 columns, not once per column
-    // beta == 1 (the trsm updates): C += v as a reduction in L2 — one
-    // add per element, rounded as c + v, with no read in the thread
+    const float alpha = float(P.alpha);
     if (P.dvec) {  // trmm: C = alpha acc + d C, d per row or per column
+        if (row >= P.m) return;
         const float drow = P.dvec_mode == 1 ? P.dvec[row] : 0.0f;
+        // 8 columns at a time: all loads of C are issued before the first is used
 #pragma unroll
         for (int c0 = 0; c0 < C::EPI_COLS; c0 += 8) {
             float cv[8];
@@ -153,36 +205,47 @@ __device__ __forceinline__ void split_store_row(const Params& P, const i64 row, 
                 Cm[row + col * P.ldc] = fmaf(d, cv[j], alpha * acc[c0 + j]);
             }
         }
-    } else if (beta == 1.0f) {
-#pragma unroll
-        for (int j = 0; j < C::EPI_COLS; ++j) {
-            const i64 col = cbase + j;
-            if (col < P.n && !(P.tri == 1 && row < col) && !(P.tri == 2 && row > col))
-                atomicAdd(Cm + row + col * P.ldc, alpha * acc[j]);
-        }
-    } else
-#pragma unroll
-    for (int c0 = 0; c0 < C::EPI_COLS; c0 += 8) {
-        float cv[8];
-        bool live[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const i64 col = cbase + c0 + j;
-            live[j] = col < P.n && !(P.tri == 1 && row < col) && !(P.tri == 2 && row > col);
-            cv[j] = (live[j] && beta != 0.0f) ? Cm[row + col * P.ldc] : 0.0f;
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            if (!live[j]) continue;
-            const float v = alpha * acc[c0 + j];
-            Cm[row + (cbase + c0 + j) * P.ldc] = (beta == 0.0f) ? v : fmaf(beta, cv[j], v);
-        }
+        return;
     }
+    int lo, hi;
+    live_columns(P, row, cbase, P.n, lo, hi);
+    split_store<C::EPI_COLS>(Cm + row + cbase * P.ldc, P.ldc, alpha, float(P.beta), acc, lo, hi);
+}
+
+// ---- one tile's reduction over the CTAs of a cluster ----------------------------------------
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t cluster_size() {
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t peer_smem(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ float4 peer_load4(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(addr)
+                 : "memory");
+    return v;
 }
 
 // Output tile `tile` of the product P, its operands' planes read through tmA / tmB (kernel
-// parameters): one CTA's whole work in the kernels below.
-template <class C>
+// parameters): one CTA's whole work in the kernels below.  CK: the CTAs of a cluster share the
+// tile, each taking an equal part of its slabs; then each leaves its sums in its own (by now
+// idle) stage buffers and adds up its share of the columns over the cluster, in the CTAs'
+// order, so results do not depend on scheduling.
+template <class C, bool CK = false>
 __device__ __forceinline__ void tc_gemm_tile(const CUtensorMap& tmA, const CUtensorMap& tmB, const Params& P,
                                              const int tile) {
     extern __shared__ uint8_t smem_raw[];
@@ -216,6 +279,11 @@ __device__ __forceinline__ void tc_gemm_tile(const CUtensorMap& tmA, const CUten
         band_slabs(P.band, m0, BM, n0, C::BN, P.band_k0, C::BK, P.num_kb, s0, s1);
         kb0 = int(s0);
         nkb = int(s1 - s0);
+    }
+    if constexpr (CK) {
+        const int S = int(cluster_size()), r = int(cluster_rank());
+        kb0 = nkb * r / S;
+        nkb = nkb * (r + 1) / S - kb0;
     }
     const int chunk_slabs = C::OZAKI ? nkb : C::CHUNK;
     const int nchunks = (nkb + chunk_slabs - 1) / chunk_slabs;
@@ -329,7 +397,15 @@ __device__ __forceinline__ void tc_gemm_tile(const CUtensorMap& tmA, const CUten
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&tempty[buf]);
             }
-            if (ok && row < P.m) split_store_row<C>(P, row, n0 + part * C::EPI_COLS, acc);
+            if constexpr (CK) {
+                // every MMA has completed, so every stage has been read; four columns of a row together
+                float4* const mine = reinterpret_cast<float4*>(smem) + part * (C::EPI_COLS / 4) * BM + quarter * 32 + lane;
+#pragma unroll
+                for (int j = 0; j < C::EPI_COLS; j += 4)
+                    mine[j / 4 * BM] = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+            } else {
+                if (ok) split_store_row<C>(P, row, n0 + part * C::EPI_COLS, acc);
+            }
         }
     }
     tc_fence_before();
@@ -339,12 +415,67 @@ __device__ __forceinline__ void tc_gemm_tile(const CUtensorMap& tmA, const CUten
         tc_fence_after();
         tmem_dealloc(tmem, C::TMEM_COLS);
     }
+    if constexpr (CK) {
+        static_assert(BM * C::BN * 4 <= C::STAGES * C::STAGE_BYTES, "the sums reuse the stage buffers");
+        __syncwarp();
+        cluster_sync_all();
+        if (warp >= 2) {
+            const int S = int(cluster_size()), r = int(cluster_rank());
+            constexpr int UNITS = C::BN / 16;
+            const int c0 = 16 * (UNITS * r / S), c1 = 16 * (UNITS * (r + 1) / S);  // this CTA's columns of the tile
+            const int quarter = warp & 3, part = (warp - 2) >> 2;
+            const i64 row = m0 + quarter * 32 + lane;
+            const uint32_t base = smem_u32(smem) + uint32_t(quarter * 32 + lane) * 16;
+            for (int c = c0 + 16 * part; c < c1; c += 16 * (C::EPI_WARPS / 4)) {
+                if (n0 + c >= P.n) break;
+                float v[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] = 0.0f;
+                for (int s0 = 0; s0 < S; s0 += 4) {  // four CTAs' loads in flight, added in order
+                    float4 t[4][4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (s0 + u < S) {
+                            const uint32_t q = peer_smem(base, uint32_t(s0 + u)) + uint32_t(c / 4 * BM * 16);
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) t[u][j] = peer_load4(q + uint32_t(j * BM * 16));
+                        }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (s0 + u < S)
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                v[4 * j] += t[u][j].x;
+                                v[4 * j + 1] += t[u][j].y;
+                                v[4 * j + 2] += t[u][j].z;
+                                v[4 * j + 3] += t[u][j].w;
+                            }
+                }
+                int lo, hi;
+                live_columns(P, row, n0 + c, P.n, lo, hi);
+                split_store<16>(static_cast<float*>(P.c) + row + (n0 + c) * P.ldc, P.ldc, float(P.alpha), float(P.beta), v,
+                                lo, hi);
+            }
+        }
+        __syncwarp();
+        cluster_sync_all();  // no CTA leaves while another reads its sums
+    }
 }
 
 template <class C>
 __global__ void __launch_bounds__(C::THREADS, 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Params P) {
     tc_gemm_tile<C>(tmA, tmB, P, int(blockIdx.x));
+}
+
+// A cluster of CTAs per tile (tc_gemm_tile, CK).  A product with fewer tiles than SMs leaves the
+// rest idle for its whole reduction, and narrower tiles fill them at a worse rate per SM
+// (launch_split_product has the figures); splitting the reduction keeps the wide tile.  The sums
+// cross the cluster through shared memory: no zeroing pass, no atomics on C, any beta.
+template <class C>
+__global__ void __launch_bounds__(C::THREADS, 1)
+tc_gemm_ck_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Params P) {
+    tc_gemm_tile<C, true>(tmA, tmB, P, int(blockIdx.x / cluster_size()));
 }
 
 // ---------------------------------------------------------------------------
@@ -822,14 +953,6 @@ struct Oz2Cfg {
     static_assert(A_PLANE % (8 * BKB) == 0 && B_PLANE % (8 * BKB) == 0, "swizzle atoms stay aligned");
 };
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 // shared::cluster address of the same variable in CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t peer_addr(const void* p, uint32_t rank) {
     uint32_t r;
@@ -1211,13 +1334,9 @@ __global__ void __launch_bounds__(256) sk_zero_kernel(Params P0, Params P1, SkWo
 template <class C>
 __device__ __forceinline__ void split_add_row(const Params& P, const i64 row, const i64 cbase,
                                               const float (&acc)[C::EPI_COLS]) {
-    float* Cm = static_cast<float*>(P.c);
-    const float alpha = float(P.alpha);
-#pragma unroll
-    for (int j = 0; j < C::EPI_COLS; ++j) {
-        const i64 col = cbase + j;
-        if (col < P.n) atomicAdd(Cm + row + col * P.ldc, alpha * acc[j]);
-    }
+    int lo, hi;
+    live_columns(P, row, cbase, P.n, lo, hi);
+    split_store<C::EPI_COLS>(static_cast<float*>(P.c) + row + cbase * P.ldc, P.ldc, float(P.alpha), 1.0f, acc, lo, hi);
 }
 
 // The split product on single CTAs, persistent over the CTA's segments (SkWork): the
@@ -1368,7 +1487,7 @@ split_sk_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant_
                 if (lane == 0) mbar_arrive(&tempty[buf]);
             }
             const i64 row = sg.m0 + quarter * 32 + lane;
-            if (!ok || row >= P.m) continue;
+            if (!ok) continue;
             const i64 cbase = sg.n0 + part * C::EPI_COLS;
             if (sg.kb0 == 0 && sg.kb1 == (sg.prod ? W.nkb1 : W.nkb0)) split_store_row<C>(P, row, cbase, acc);
             else split_add_row<C>(P, row, cbase, acc);
@@ -1772,6 +1891,57 @@ int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, Params& P, const cha
     return check_launch(name);
 }
 
+// Launch attributes of tc_gemm_ck_kernel with S CTAs per cluster.
+struct CkLaunch {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+    CkLaunch(unsigned ctas, int S, int threads, int smem, cudaStream_t s) {
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = unsigned(S);
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.gridDim = dim3(ctas);
+        cfg.blockDim = dim3(unsigned(threads));
+        cfg.dynamicSmemBytes = size_t(smem);
+        cfg.stream = s;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+    }
+};
+constexpr int CK_MAX = 8;  // CTAs per cluster (portable)
+
+// Clusters of S CTAs of tc_gemm_ck_kernel<C> that can be resident at once (0: none), cached
+// per device.
+template <class C>
+int ck_clusters(int dev, int S) {
+    static std::atomic<int> cache[64][CK_MAX + 1];  // count + 1
+    if (dev < 0 || dev >= 64) return 0;
+    int v = cache[dev][S].load();
+    if (!v) {
+        int n = 0;
+        const CkLaunch l(unsigned(S), S, C::THREADS, C::SMEM_BYTES, nullptr);
+        if (cudaFuncSetAttribute(tc_gemm_ck_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES) !=
+                cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, tc_gemm_ck_kernel<C>, &l.cfg) != cudaSuccess) {
+            cudaGetLastError();
+            n = 0;
+        }
+        v = n + 1;
+        cache[dev][S].store(v);
+    }
+    return v - 1;
+}
+
+template <class C>
+int launch_ck(const CUtensorMap& ma, const CUtensorMap& mb, Params& P, int S, const char* name) {
+    P.err = device_error_flag();
+    const i64 ctas = i64(P.tiles_m) * P.tiles_n * S;
+    if (ctas > 0x7fffffff) return MBG_ERR_UNSUPPORTED;
+    ProfScope prof(name);
+    const CkLaunch l(unsigned(ctas), S, C::THREADS, C::SMEM_BYTES, stream());
+    MBG_CUDA(cudaLaunchKernelEx(&l.cfg, tc_gemm_ck_kernel<C>, ma, mb, P));
+    return check_launch(name);
+}
+
 // CTAs of split_sk_kernel that can be resident at once on this device (one per SM),
 // cached per device.
 template <class C>
@@ -1870,35 +2040,66 @@ int launch_sk(const CUtensorMap* ma, const CUtensorMap* mb, Params* P, int nprod
     return check_launch(name);
 }
 
+// Tiles of 128 x bn that the triangle mask keeps.
+inline i64 live_tiles(const Params& P, int bn) {
+    const i64 tn_all = cdiv(P.n, bn);
+    if (!P.tri) return i64(P.tiles_m) * tn_all;
+    i64 live = 0;
+    for (i64 tm = 0; tm < P.tiles_m; ++tm)
+        for (i64 tn = 0; tn < tn_all; ++tn) {
+            const i64 m0 = tm * BM, n0 = tn * bn;
+            if (P.tri == 1 && m0 + BM <= n0) continue;
+            if (P.tri == 2 && m0 > n0 + bn - 1) continue;
+            ++live;
+        }
+    return live;
+}
+
+// Tile width and CTAs per tile of a split product, by the estimated time in microseconds of its
+// waves: a CTA's start and end, and its 32-deep slabs, which take longer the more of the chip
+// reads planes at once.  Measured for six products (slabs of 128 x 256 / 128 / 64 tiles): 0.76,
+// 0.55 and 0.55 on a few SMs, 1.18 at 8192^3 for the widest; a narrow tile reads more
+// operand bytes per flop.  Three products take 0.6 of that.  A cluster of S that shares a tile adds
+// 2 + 0.7 S for its launch and the exchange of its sums.  (875 x 736 x 1480: 35 us on 42 tiles of
+// 128 x 128, 23 with three CTAs each; 512^3: 17.3 against 14.9 with three or four.)
+struct SplitShape {
+    int bn, S;
+};
+template <class Wide, class Mid>
+SplitShape split_shape(const Params& P, int terms, int dev, int sms) {
+    const double scale = terms == 3 ? 1.0 : 0.6;
+    SplitShape best{256, 1};
+    double t_best = 0;
+    for (int bn = 256; bn >= 64; bn /= 2) {
+        const i64 tiles = imax(1, live_tiles(P, bn));
+        for (int S = 1; S <= (bn >= 128 && P.band == KB_NONE && !P.dvec ? CK_MAX : 1) && S <= P.num_kb; ++S) {
+            const i64 room = S == 1 ? sms : bn == 256 ? ck_clusters<Wide>(dev, S) : ck_clusters<Mid>(dev, S);
+            if (room <= 0) continue;
+            const double busy = double(imin(tiles, room) * S) / sms;
+            const double slab = scale * (bn == 256 ? 0.76 + 0.42 * busy : bn == 128 ? 0.48 + 0.31 * busy : 0.55 + 0.06 * busy);
+            const double fixed = bn == 256 ? 6.0 : 3.5;
+            const double t = double(cdiv(tiles, room)) * (fixed + double(cdiv(P.num_kb, S)) * slab + (S > 1 ? 2.0 + 0.7 * S : 0.0));
+            if (t_best == 0 || t < t_best) {
+                t_best = t;
+                best = SplitShape{bn, S};
+            }
+        }
+    }
+    return best;
+}
+
 // The split product on planes pa (op(A), a_rows rows from pa, planes a_plane_rows apart)
-// and pb (op(B)^T, b_rows rows): 128 x 256 tiles (a 128 x 128 tile's MMAs read a third
-// more operand bytes per flop from shared memory, so the wide tile wins wherever it fills
-// more than half of the SMs); 128 x 128 when the wide ones would fill at most half, 128 x 64
-// at most a quarter (counting, under a triangle mask, only the tiles it keeps).  More wide tiles than SMs with a last wave mostly empty (beta = 0, no
-// band, mask or d-vector): split_sk_kernel with a stream-K tail.  Sets the B map and
-// P.tiles_n.
+// and pb (op(B)^T, b_rows rows).  More wide tiles than SMs with a last wave mostly empty (beta = 0,
+// no band, mask or d-vector): split_sk_kernel with a stream-K tail; else the shape that
+// split_shape takes to be fastest.  Sets the B map and P.tiles_n.
 int launch_split_product(int terms, const __nv_bfloat16* pa, i64 a_rows, i64 a_plane_rows, const __nv_bfloat16* pb,
                          i64 b_rows, i64 Kp, Params& P) {
     int dev = 0, sms = 148;
     MBG_CUDA(cudaGetDevice(&dev));
     MBG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    i64 wide_tiles = i64(P.tiles_m) * cdiv(P.n, 256);
-    if (P.tri) {  // only the tiles the triangle mask keeps do work
-        i64 live = 0;
-        for (i64 tm = 0; tm < P.tiles_m; ++tm)
-            for (i64 tn = 0; tn < cdiv(P.n, 256); ++tn) {
-                const i64 m0 = tm * BM, n0 = tn * 256;
-                if (P.tri == 1 && m0 + BM <= n0) continue;
-                if (P.tri == 2 && m0 > n0 + 255) continue;
-                ++live;
-            }
-        wide_tiles = live;
-    }
-    const int bn = 4 * wide_tiles <= sms ? 64 : (2 * wide_tiles <= sms ? 128 : 256);
     CUtensorMap ma, mb;
     MBG_TRY(make_map(&ma, pa, false, Kp, a_rows, terms, 64, BM, a_plane_rows));
-    if (bn == 256 && wide_tiles > sms && P.beta == 0.0 && !P.tri && P.band == KB_NONE && !P.dvec) {
-        // more wide tiles than SMs and a last wave mostly empty: persistent, stream-K tail
+    if (i64(P.tiles_m) * cdiv(P.n, 256) > sms && P.beta == 0.0 && !P.tri && P.band == KB_NONE && !P.dvec) {
         MBG_TRY(make_map(&mb, pb, false, Kp, b_rows, terms, 64, 256));
         P.tiles_n = int(cdiv(P.n, 256));
         const CUtensorMap mas[2] = {ma, ma}, mbs[2] = {mb, mb};
@@ -1908,16 +2109,24 @@ int launch_split_product(int terms, const __nv_bfloat16* pa, i64 a_rows, i64 a_p
                                   : launch_sk<CfgBF16x6>(mas, mbs, Ps, 1, true, "tc_gemm_bf16x6", &declined);
         if (st || !declined) return st;
     }
-    MBG_TRY(make_map(&mb, pb, false, Kp, b_rows, terms, 64, bn));
-    P.tiles_n = int(cdiv(P.n, bn));
+    const SplitShape sh = terms == 2 ? split_shape<CfgBF16x3, CfgBF16x3m>(P, terms, dev, sms)
+                                     : split_shape<CfgBF16x6, CfgBF16x6m>(P, terms, dev, sms);
+    MBG_TRY(make_map(&mb, pb, false, Kp, b_rows, terms, 64, sh.bn));
+    P.tiles_n = int(cdiv(P.n, sh.bn));
     if (terms == 2) {
-        if (bn == 64) return launch_tc<CfgBF16x3n>(ma, mb, P, "tc_gemm_bf16x3");
-        if (bn == 128) return launch_tc<CfgBF16x3m>(ma, mb, P, "tc_gemm_bf16x3");
-        return launch_tc<CfgBF16x3>(ma, mb, P, "tc_gemm_bf16x3");
+        if (sh.bn == 64) return launch_tc<CfgBF16x3n>(ma, mb, P, "tc_gemm_bf16x3");
+        if (sh.bn == 128)
+            return sh.S > 1 ? launch_ck<CfgBF16x3m>(ma, mb, P, sh.S, "tc_gemm_bf16x3")
+                            : launch_tc<CfgBF16x3m>(ma, mb, P, "tc_gemm_bf16x3");
+        return sh.S > 1 ? launch_ck<CfgBF16x3>(ma, mb, P, sh.S, "tc_gemm_bf16x3")
+                        : launch_tc<CfgBF16x3>(ma, mb, P, "tc_gemm_bf16x3");
     }
-    if (bn == 64) return launch_tc<CfgBF16x6n>(ma, mb, P, "tc_gemm_bf16x6");
-    if (bn == 128) return launch_tc<CfgBF16x6m>(ma, mb, P, "tc_gemm_bf16x6");
-    return launch_tc<CfgBF16x6>(ma, mb, P, "tc_gemm_bf16x6");
+    if (sh.bn == 64) return launch_tc<CfgBF16x6n>(ma, mb, P, "tc_gemm_bf16x6");
+    if (sh.bn == 128)
+        return sh.S > 1 ? launch_ck<CfgBF16x6m>(ma, mb, P, sh.S, "tc_gemm_bf16x6")
+                        : launch_tc<CfgBF16x6m>(ma, mb, P, "tc_gemm_bf16x6");
+    return sh.S > 1 ? launch_ck<CfgBF16x6>(ma, mb, P, sh.S, "tc_gemm_bf16x6")
+                    : launch_tc<CfgBF16x6>(ma, mb, P, "tc_gemm_bf16x6");
 }
 
 template <int TERMS>

@@ -19,6 +19,7 @@
 // m-contiguous operand, [m][k] rows of 36 doubles for a k-contiguous one.  Both
 // paddings make the fragment loads A[row = lane / 4][k = lane % 4] and
 // B[k = lane % 4][col = lane / 4] two wavefronts each, the minimum for 256 bytes.
+#include "cluster.cuh"
 #include "mbg_internal.cuh"
 
 namespace mbg {
@@ -67,11 +68,17 @@ struct DmmaCfg {
     static constexpr int A_ELEMS = (DK * (BM + 8) > BM * DKP) ? DK * (BM + 8) : BM * DKP;
     static constexpr int B_ELEMS = (DK * (BN + 8) > BN * DKP) ? DK * (BN + 8) : BN * DKP;
     static constexpr size_t SMEM = sizeof(double) * size_t(DSTAGES) * (A_ELEMS + B_ELEMS);
+    // a shared tile's sums, [column][row]: the pad spreads a fragment's columns over the banks
+    static constexpr int LSUM = BM + 2;
+    static_assert(sizeof(double) * size_t(LSUM) * BN <= SMEM, "the sums reuse the stages");
 };
 
 // VEC = 2: both operands 16-byte aligned with even leading dimensions, so pairs
 // of elements along the contiguous index are copied 16 bytes at a time.
-template <class C, bool TA, bool TB, int TRI, int BM, int BN, int VEC>
+// CK: the CTAs of a cluster share a tile, each taking an equal part of its slabs; each then leaves
+// its sums in its shared memory and adds up its share of the columns over the cluster, in the
+// CTAs' order, so results do not depend on scheduling.
+template <class C, bool TA, bool TB, int TRI, int BM, int BN, int VEC, bool CK = false>
 __global__ void __launch_bounds__(C::THREADS, 1)
 gemm_dmma_kernel(i64 m, i64 n, i64 k, double alpha, const double* __restrict__ A, i64 lda,
                  const double* __restrict__ B, i64 ldb, double beta, double* __restrict__ Cm, i64 ldc, int band) {
@@ -83,7 +90,7 @@ gemm_dmma_kernel(i64 m, i64 n, i64 k, double alpha, const double* __restrict__ A
 
     i64 tm, tn;
     if (TRI == 0) {
-        tm = blockIdx.x;
+        tm = CK ? blockIdx.x / clu::size() : blockIdx.x;
         tn = blockIdx.y;
         band_order(band, tm, tn);
     } else {
@@ -146,6 +153,11 @@ gemm_dmma_kernel(i64 m, i64 n, i64 k, double alpha, const double* __restrict__ A
     // slabs [kt0, kt0 + nk) of the reduction: all of them, or the tile's band
     i64 kt0 = 0, kt1 = (k + DK - 1) / DK;
     if (band != KB_NONE) band_slabs(band, m0, BM, n0, BN, 0, DK, kt1, kt0, kt1);
+    if constexpr (CK) {
+        const i64 all = kt1, S = clu::size(), r = clu::rank();
+        kt0 = all * r / S;
+        kt1 = all * (r + 1) / S;
+    }
     const i64 nk = kt1 - kt0;
 #pragma unroll
     for (int s = 0; s < DSTAGES - 1; ++s) {
@@ -176,6 +188,45 @@ gemm_dmma_kernel(i64 m, i64 n, i64 k, double alpha, const double* __restrict__ A
     }
     cp_wait<0>();
 
+    if constexpr (CK) {
+        __syncthreads();  // every warp has read the last slab
+#pragma unroll
+        for (int i = 0; i < C::MI; ++i)
+#pragma unroll
+            for (int j = 0; j < C::NJ; ++j)
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+                    dsm[(wn0 + 8 * j + 2 * lk + e) * C::LSUM + wm0 + 8 * i + lr] = acc[i][j][e];
+        clu::sync_all();
+        const int S = int(clu::size()), r = int(clu::rank());
+        const int c0 = BN * r / S, c1 = BN * (r + 1) / S;
+        constexpr int PAIRS = BM / 2;
+        const int row = 2 * (tid % PAIRS);
+        const unsigned base = (unsigned)__cvta_generic_to_shared(dsm + row);
+        for (int cj = c0 + tid / PAIRS; cj < c1 && n0 + cj < n; cj += C::THREADS / PAIRS) {
+            double v[2] = {0.0, 0.0};
+            for (int s0 = 0; s0 < S; s0 += 4) {  // four CTAs' loads in flight, added in order
+                double2 t[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (s0 + u < S) t[u] = clu::load2(clu::peer(base, unsigned(s0 + u)) + unsigned(cj * C::LSUM * 8));
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (s0 + u < S) { v[0] += t[u].x; v[1] += t[u].y; }
+            }
+            double* cp = Cm + m0 + row + (n0 + cj) * ldc;
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+                if (m0 + row + i < m) {
+                    const double w = alpha * v[i];
+                    if (beta == 0.0) cp[i] = w;
+                    else if (beta == 1.0) atomicAdd(cp + i, w);
+                    else cp[i] = fma(beta, cp[i], w);
+                }
+        }
+        clu::sync_all();  // no CTA leaves while another reads its sums
+        return;
+    }
     // D fragment: row lane / 4, columns 2 (lane % 4) + {0, 1}
 #pragma unroll
     for (int i = 0; i < C::MI; ++i) {
@@ -245,6 +296,59 @@ int launch_dmma(bool ta, bool tb, dim3 grid, i64 m, i64 n, i64 k, double alpha, 
     return launch_dmma_v<C, TRI, BM, BN, 1>(ta, tb, grid, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc, band);
 }
 
+template <bool TA, bool TB, int VEC>
+int launch_dmma_ck_t(int S, i64 m, i64 n, i64 k, double alpha, const double* a, i64 lda, const double* b, i64 ldb,
+                     double beta, double* c, i64 ldc) {
+    auto kern = gemm_dmma_kernel<Small, TA, TB, 0, 64, 64, VEC, true>;
+    static std::atomic<unsigned> configured{0};  // one bit per device
+    int dev = 0;
+    MBG_CUDA(cudaGetDevice(&dev));
+    if (!configured_on(configured, dev)) {
+        MBG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Small::SMEM));
+        mark_configured(configured, dev);
+    }
+    clu::Launch l(unsigned(cdiv(m, 64)) * unsigned(S), S, Small::THREADS, Small::SMEM, stream());
+    l.cfg.gridDim.y = unsigned(cdiv(n, 64));
+    MBG_CUDA(cudaLaunchKernelEx(&l.cfg, kern, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc, int(KB_NONE)));
+    return check_launch("gemm_dmma_f64");
+}
+
+int launch_dmma_ck(int S, bool ta, bool tb, i64 m, i64 n, i64 k, double alpha, const double* a, i64 lda,
+                   const double* b, i64 ldb, double beta, double* c, i64 ldc) {
+    const bool vec = (reinterpret_cast<uintptr_t>(a) % 16 == 0) && (reinterpret_cast<uintptr_t>(b) % 16 == 0) &&
+                     lda % 2 == 0 && ldb % 2 == 0;
+#define DMC(TA_, TB_) \
+    return vec ? launch_dmma_ck_t<TA_, TB_, 2>(S, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc) \
+               : launch_dmma_ck_t<TA_, TB_, 1>(S, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc)
+    if (!ta && !tb) DMC(false, false);
+    if (!ta) DMC(false, true);
+    if (!tb) DMC(true, false);
+    DMC(true, true);
+#undef DMC
+}
+
+// CTAs per 64 x 64 tile, by the estimated time in microseconds: a 32-deep slab takes 1.7 for a
+// CTA alone on its SM (latency) and 2.3 for the two that fit together (the FP64 pipe's rate);
+// sharing a tile adds 1 + 0.2 S, and has to be worth a tenth.  (Measured around each call, launch
+// included: 300 x 521 x 257 TN 25 us, 17 with three CTAs per tile; 512^3 NT 35, 25 with two and 21
+// with four; 64 x 64 x 1000 TT 58, 17 with eight; 1024 x 1024 x 512 NT 50, 60 with two.)
+inline int dmma_share(i64 m, i64 n, i64 k) {
+    const i64 slabs = cdiv(k, DK), tiles = cdiv(m, 64) * cdiv(n, 64);
+    int best = 1;
+    double t_best = 0;
+    for (int S = 1; S <= clu::MAX_CTAS && S <= slabs; ++S) {
+        const i64 per_sm = cdiv(tiles * S, clu::usable_sms(S));
+        const double slab = 2.3 * double(per_sm / 2) + 1.7 * double(per_sm % 2);
+        double t = double(cdiv(slabs, S)) * slab + (S > 1 ? 1.0 + 0.2 * S : 0.0);
+        if (S > 1) t *= 1.1;
+        if (t_best == 0 || t < t_best) {
+            t_best = t;
+            best = S;
+        }
+    }
+    return best;
+}
+
 }  // namespace
 
 // C := alpha op(A) op(B) + beta C in FP64 on the tensor pipe (alpha != 0, k > 0).
@@ -256,6 +360,8 @@ int dgemm_dmma(char ta, char tb, i64 m, i64 n, i64 k, double alpha, const double
     if (gm * gn < 2 * 148) {  // under two waves of 128 x 128 tiles: 64 x 64 tiles
         const i64 sm = cdiv(m, 64), sn = cdiv(n, 64);
         if (sn > 65535 || sm > 0x7fffffff) return MBG_ERR_UNSUPPORTED;
+        const int S = band == KB_NONE ? dmma_share(m, n, k) : 1;
+        if (S > 1) return launch_dmma_ck(S, is_t(ta), is_t(tb), m, n, k, alpha, a, lda, b, ldb, beta, c, ldc);
         return launch_dmma<Small, 0, 64, 64>(is_t(ta), is_t(tb), dim3((unsigned)sm, (unsigned)sn), m, n, k, alpha,
                                              a, lda, b, ldb, beta, c, ldc, band);
     }

@@ -3,8 +3,8 @@
 // :2092-2436) and, with a triangular tile schedule, ssyrk
 // (src/level3/syrk.mojo:20-200).
 //
-// One CTA per 128 x 128 tile of C, or per 64 x 64 tile for launches that would
-// fill fewer than two waves of 128-tiles; the tile code (cp.async pipeline,
+// One CTA per 128 x 128 tile of C; launches that would fill fewer than two waves of those
+// may take 64 x 64 tiles and a cluster of CTAs per tile; the tile code (cp.async pipeline,
 // register blocking, epilogue) is gemm_f32_tile.cuh, shared with the grouped
 // sgemm plans.
 #include "mbg_internal.cuh"
@@ -34,6 +34,93 @@ gemm_f32_kernel(i64 m, i64 n, i64 k, float alpha, const float* __restrict__ A, i
     f32_tile<FT, TA, TB, TRI, VA, VB>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tm, tn, fsm, band);
 }
 
+
+// A cluster of CTAs per tile (f32_tile, CK): a product with few tiles spreads its reduction
+// over the SMs they leave idle.
+template <int FT, bool TA, bool TB, bool VA, bool VB>
+__global__ void __launch_bounds__(FNT, FT == 128 ? 2 : 4)
+gemm_f32_ck_kernel(i64 m, i64 n, i64 k, float alpha, const float* __restrict__ A, i64 lda,
+                   const float* __restrict__ B, i64 ldb, float beta, float* __restrict__ C, i64 ldc, unsigned tiles_m) {
+    extern __shared__ __align__(16) float fsm[];
+    const unsigned tile = blockIdx.x / clu::size();
+    f32_tile<FT, TA, TB, 0, VA, VB, true>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tile % tiles_m, tile / tiles_m,
+                                          fsm);
+}
+
+template <int FT, bool TA, bool TB, bool VA, bool VB>
+int launch_f32_ck_t(int S, i64 m, i64 n, i64 k, float alpha, const float* a, i64 lda, const float* b, i64 ldb,
+                    float beta, float* c, i64 ldc) {
+    constexpr size_t SM = f32_ck_smem<FT>();
+    static std::atomic<unsigned> configured{0};  // one bit per device
+    int dev = 0;
+    MBG_CUDA(cudaGetDevice(&dev));
+    if (!configured_on(configured, dev)) {
+        MBG_CUDA(cudaFuncSetAttribute(gemm_f32_ck_kernel<FT, TA, TB, VA, VB>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM));
+        mark_configured(configured, dev);
+    }
+    const unsigned gm = unsigned(cdiv(m, FT));
+    const clu::Launch l(gm * unsigned(cdiv(n, FT)) * unsigned(S), S, FNT, SM, stream());
+    MBG_CUDA(cudaLaunchKernelEx(&l.cfg, gemm_f32_ck_kernel<FT, TA, TB, VA, VB>, m, n, k, alpha, a, lda, b, ldb, beta,
+                                c, ldc, gm));
+    return check_launch("gemm_f32");
+}
+
+template <int FT>
+int launch_f32_ck(int S, bool ta, bool tb, i64 m, i64 n, i64 k, float alpha, const float* a, i64 lda, const float* b,
+                  i64 ldb, float beta, float* c, i64 ldc) {
+    const bool va = f32_vec(!ta, a, lda), vb = f32_vec(tb, b, ldb);
+#define CKL(TA_, TB_, VA_, VB_) \
+    return launch_f32_ck_t<FT, TA_, TB_, VA_, VB_>(S, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc)
+    if (!ta && tb) {
+        if (va && vb) CKL(false, true, true, true);
+        if (va) CKL(false, true, true, false);
+        if (vb) CKL(false, true, false, true);
+        CKL(false, true, false, false);
+    }
+    if (!ta) {
+        if (va) CKL(false, false, true, false);
+        CKL(false, false, false, false);
+    }
+    if (tb) {
+        if (vb) CKL(true, true, false, true);
+        CKL(true, true, false, false);
+    }
+    CKL(true, false, false, false);
+#undef CKL
+}
+
+// Tile and CTAs per tile of a product under two waves of 128-tiles, by the estimated time in
+// microseconds.  A 16-deep slab takes the longer of a CTA's own latency and its share of the SM:
+// 0.51 and 0.46 for 64-tiles, 1.54 for 128-tiles, and 0.74, 0.64 and 1.76 where neither operand
+// takes 16-byte copies; sharing a tile adds 1 + 0.2 S, and has to be worth a tenth.  (Measured
+// around each call, launch included: 512^3 NT 26.9 us on 64-tiles, 17.7 with four CTAs each, 19.6 on
+// 128-tiles with six; 64 x 64 x 1000 TT 54.9 and, with eight, 14.7; 1000^3 NN 91 on 64-tiles, 68 on
+// 128-tiles with two.)
+struct F32Shape {
+    int ft, S;
+};
+inline F32Shape f32_shape(i64 m, i64 n, i64 k, int vec_operands, bool may_share) {
+    F32Shape best{64, 1};
+    double t_best = 0;
+    const i64 slabs = cdiv(k, FK);
+    const double scalar = (2 - vec_operands) / 2.0;
+    for (int ft = 64; ft <= 128; ft *= 2) {
+        const i64 tiles = cdiv(m, ft) * cdiv(n, ft);
+        const double lat = ft == 128 ? 1.54 + 0.22 * scalar : 0.51 + 0.23 * scalar;
+        const double rate = ft == 128 ? lat : 0.46 + 0.18 * scalar;
+        for (int S = 1; S <= (may_share ? clu::MAX_CTAS : 1) && S <= slabs; ++S) {
+            const double share = rate * double(cdiv(tiles * S, clu::usable_sms(S)));
+            double t = double(cdiv(slabs, S)) * (share > lat ? share : lat) + (S > 1 ? 1.0 + 0.2 * S : 0.0);
+            if (ft == 128 || S > 1) t *= 1.1;
+            if (t_best == 0 || t < t_best) {
+                t_best = t;
+                best = F32Shape{ft, S};
+            }
+        }
+    }
+    return best;
+}
 
 template <int FT, int TRI, bool VA, bool VB>
 int launch_f32_v(bool ta, bool tb, dim3 grid, i64 m, i64 n, i64 k, float alpha, const float* a, i64 lda,
@@ -104,8 +191,8 @@ int launch_f32_transpose(i64 rows, i64 cols, const float* src, i64 lds, float* d
 
 }  // namespace
 
-// C := alpha op(A) op(B) + beta C (alpha != 0, k > 0): 128 x 128 tiles, or 64 x 64
-// tiles (4 x 4 per thread) when 128-tiles would fill fewer than two waves.
+// C := alpha op(A) op(B) + beta C (alpha != 0, k > 0): 128 x 128 tiles, or, when those would
+// fill fewer than two waves, the tile and the CTAs per tile that f32_shape takes to be fastest.
 // band (KB_*): one operand is a dense triangle; each tile runs its part of k.
 // The tiles copy an operand 16 bytes at a time only when it is contiguous along m
 // (op(A)) or n (op(B)), as in NT.  In a large call (m n k >= 2^30) an operand that is
@@ -136,7 +223,13 @@ int sgemm_f32(char ta, char tb, i64 m, i64 n, i64 k, float alpha, const float* a
     }
     ProfScope prof("gemm_f32");
     const i64 gm = cdiv(m, 128), gn = cdiv(n, 128);
-    if (gm * gn < 2 * 148) {
+    const F32Shape sh = gm * gn >= 2 * 148 ? F32Shape{128, 1}
+                                           : f32_shape(m, n, k, f32_vec(is_n(ta), a, lda) + f32_vec(is_t(tb), b, ldb),
+                                                       band == KB_NONE);
+    if (sh.S > 1)
+        return sh.ft == 128 ? launch_f32_ck<128>(sh.S, is_t(ta), is_t(tb), m, n, k, alpha, a, lda, b, ldb, beta, c, ldc)
+                            : launch_f32_ck<64>(sh.S, is_t(ta), is_t(tb), m, n, k, alpha, a, lda, b, ldb, beta, c, ldc);
+    if (sh.ft == 64) {
         const i64 sm = cdiv(m, 64), sn = cdiv(n, 64);
         if (sn > 65535 || sm > 0x7fffffff) return MBG_ERR_UNSUPPORTED;
         return launch_f32<64, 0>(is_t(ta), is_t(tb), dim3((unsigned)sm, (unsigned)sn), m, n, k, alpha, a, lda, b,

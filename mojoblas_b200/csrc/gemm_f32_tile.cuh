@@ -14,6 +14,7 @@
 // as fma(1, c, v)).
 #pragma once
 
+#include "cluster.cuh"
 #include "mbg_internal.cuh"
 
 namespace mbg {
@@ -91,7 +92,10 @@ __device__ __forceinline__ void f32_stage(float* tile, const float* __restrict__
 // One FT x FT tile (tm, tn) of C := alpha op(A) op(B) + beta C by the whole CTA,
 // staging through `fsm` (f32_smem<FT>() bytes); every copy it issued has landed
 // when it returns.  band (KB_*): one operand triangular, only the tile's slabs run.
-template <int FT, bool TA, bool TB, int TRI, bool VA, bool VB>
+// CK: the CTAs of a cluster share the tile, each taking an equal part of the slabs; each then
+// leaves its sums in its shared memory (f32_ck_smem<FT>() bytes in all) and adds up its share
+// of the columns over the cluster, in the CTAs' order, so results do not depend on scheduling.
+template <int FT, bool TA, bool TB, int TRI, bool VA, bool VB, bool CK = false>
 __device__ __forceinline__ void f32_tile(i64 m, i64 n, i64 k, float alpha, const float* __restrict__ A, i64 lda,
                                          const float* __restrict__ B, i64 ldb, float beta, float* __restrict__ C,
                                          i64 ldc, i64 tm, i64 tn, float* fsm, int band = KB_NONE) {
@@ -117,6 +121,11 @@ __device__ __forceinline__ void f32_tile(i64 m, i64 n, i64 k, float alpha, const
     // slabs [kt0, kt0 + nk) of the reduction: all of them, or the tile's band
     i64 kt0 = 0, kt1 = (k + FK - 1) / FK;
     if (band != KB_NONE) band_slabs(band, m0, FT, n0, FT, 0, FK, kt1, kt0, kt1);
+    if constexpr (CK) {
+        const i64 all = kt1, S = clu::size(), r = clu::rank();
+        kt0 = all * r / S;
+        kt1 = all * (r + 1) / S;
+    }
     const i64 nk = kt1 - kt0;
 #pragma unroll
     for (int s = 0; s < FSTAGES - 1; ++s) {
@@ -162,6 +171,51 @@ __device__ __forceinline__ void f32_tile(i64 m, i64 n, i64 k, float alpha, const
 #pragma unroll
         for (int j = 0; j < TM / 2; ++j) f2_unpack(accp[i][j], acc[i][2 * j], acc[i][2 * j + 1]);
 
+    if constexpr (CK) {
+        __syncthreads();  // every thread has read the last slab: the sums take its place, [column][row]
+#pragma unroll
+        for (int j = 0; j < TM; ++j) {
+            const int cj = j < 4 ? ty * 4 + j : 64 + ty * 4 + (j - 4);
+#pragma unroll
+            for (int i = 0; i < TM; i += 4)
+                *reinterpret_cast<float4*>(fsm + cj * FT + (i ? 64 : 0) + tx * 4) =
+                    make_float4(acc[i][j], acc[i + 1][j], acc[i + 2][j], acc[i + 3][j]);
+        }
+        clu::sync_all();
+        const int S = int(clu::size()), r = int(clu::rank());
+        const int c0 = FT * r / S, c1 = FT * (r + 1) / S;
+        constexpr int QUADS = FT / 4;
+        const int row = 4 * (tid % QUADS);
+        const unsigned base = (unsigned)__cvta_generic_to_shared(fsm + row);
+        const bool whole = m0 + row + 4 <= m && ldc % 4 == 0 && reinterpret_cast<uintptr_t>(C) % 16 == 0;
+        for (int cj = c0 + tid / QUADS; cj < c1 && n0 + cj < n; cj += FNT / QUADS) {
+            float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            for (int s0 = 0; s0 < S; s0 += 4) {  // four CTAs' loads in flight, added in order
+                float4 t[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (s0 + u < S) t[u] = clu::load4(clu::peer(base, unsigned(s0 + u)) + unsigned(cj * FT * 4));
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (s0 + u < S) { v[0] += t[u].x; v[1] += t[u].y; v[2] += t[u].z; v[3] += t[u].w; }
+            }
+            float* cp = C + m0 + row + (n0 + cj) * ldc;
+            if (whole && beta == 0.0f) {
+                *reinterpret_cast<float4*>(cp) = make_float4(alpha * v[0], alpha * v[1], alpha * v[2], alpha * v[3]);
+                continue;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (m0 + row + i < m) {
+                    const float w = alpha * v[i];
+                    if (beta == 0.0f) cp[i] = w;
+                    else if (beta == 1.0f) atomicAdd(cp + i, w);
+                    else cp[i] = fmaf(beta, cp[i], w);
+                }
+        }
+        clu::sync_all();  // no CTA leaves while another reads its sums
+        return;
+    }
 #pragma unroll
     for (int j = 0; j < TM; ++j) {
         const i64 gj = n0 + (j < 4 ? ty * 4 + j : 64 + ty * 4 + (j - 4));
@@ -189,6 +243,9 @@ __device__ __forceinline__ void f32_tile(i64 m, i64 n, i64 k, float alpha, const
 
 template <int FT>
 constexpr size_t f32_smem() { return sizeof(float) * size_t(FSTAGES) * FK * FTile<FT>::LD * 2; }
+
+template <int FT>
+constexpr size_t f32_ck_smem() { return f32_smem<FT>() > sizeof(float) * FT * FT ? f32_smem<FT>() : sizeof(float) * FT * FT; }
 
 // 16-byte copies need the operand contiguous along m (n), a 16-byte aligned base and ld % 4 == 0
 __host__ __device__ inline bool f32_vec(bool contiguous_rows, const float* p, i64 ld) {

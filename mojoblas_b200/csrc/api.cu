@@ -190,6 +190,7 @@ static int gemm_host_pipelined(int mode, int slices, char ta, char tb, i64 m, i6
     if (hb) { MBG_TRY(wb.reserve(e * size_t(br) * size_t(bc))); db = wb.as<T>(); dldb = br; }
     if (hc) { MBG_TRY(wc.reserve(e * size_t(m) * size_t(n))); dc = wc.as<T>(); dldc = m; }
 
+    const ScheduleColumns whole(n);
     const std::vector<i64> widths = pipeline_widths(n);
     struct Guard {  // on every return: the copy streams' work is ordered before the library stream's
         std::vector<cudaEvent_t> v;   // next use of the workspace blocks, then the events are destroyed

@@ -222,10 +222,12 @@ int sgemm_f32(char ta, char tb, i64 m, i64 n, i64 k, float alpha, const float* a
         return sgemm_f32(ta, tb, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc, band);
     }
     ProfScope prof("gemm_f32");
-    const i64 gm = cdiv(m, 128), gn = cdiv(n, 128);
-    const F32Shape sh = gm * gn >= 2 * 148 ? F32Shape{128, 1}
-                                           : f32_shape(m, n, k, f32_vec(is_n(ta), a, lda) + f32_vec(is_t(tb), b, ldb),
-                                                       band == KB_NONE);
+    const i64 gm = cdiv(m, 128), gn = cdiv(n, 128), ns = schedule_columns(n);
+    // (what the pipelined host path takes is scheduled alike whatever the operands' alignment: its
+    // staged copies have leading dimensions of their own)
+    const int vec = double(m) * double(ns) * double(k) >= double(1ll << 34)
+                        ? 2 : int(f32_vec(is_n(ta), a, lda)) + int(f32_vec(is_t(tb), b, ldb));
+    const F32Shape sh = gm * cdiv(ns, 128) >= 2 * 148 ? F32Shape{128, 1} : f32_shape(m, ns, k, vec, band == KB_NONE);
     if (sh.S > 1)
         return sh.ft == 128 ? launch_f32_ck<128>(sh.S, is_t(ta), is_t(tb), m, n, k, alpha, a, lda, b, ldb, beta, c, ldc)
                             : launch_f32_ck<64>(sh.S, is_t(ta), is_t(tb), m, n, k, alpha, a, lda, b, ldb, beta, c, ldc);

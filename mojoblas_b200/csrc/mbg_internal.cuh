@@ -77,6 +77,17 @@ struct StreamScope {
     StreamScope& operator=(const StreamScope&) = delete;
 };
 
+// The pipelined host path computes a product in column blocks.  Whether, and into how many parts,
+// a reduction is divided depends on the size of the product, and has to be the same for every
+// block as for one call on device pointers, or the sums would be rounded differently: for its
+// lifetime, schedules of the calling thread's products go by `n` columns.
+struct ScheduleColumns {
+    explicit ScheduleColumns(i64 n);
+    ~ScheduleColumns();
+    ScheduleColumns(const ScheduleColumns&) = delete;
+};
+i64 schedule_columns(i64 n);  // the columns to schedule for: the scope's, or n
+
 // Two non-blocking streams of the current device (host->device and device->host
 // copies of the pipelined host path), created on first use and kept.
 int copy_streams(cudaStream_t* in, cudaStream_t* out);

@@ -19,6 +19,7 @@ cudaStream_t g_stream = nullptr;               // mbg_set_stream: the process-wi
 thread_local cudaStream_t t_stream = nullptr;  // mbg_set_thread_stream: this thread's override
 thread_local bool t_stream_on = false;
 std::atomic<bool> g_sync{true};
+thread_local i64 t_schedule_columns = 0;      // ScheduleColumns: 0 outside its scope
 thread_local std::string g_last_error;
 std::atomic<int> g_fail_alloc_countdown{0};
 std::atomic<int64_t> g_launches{0};
@@ -205,6 +206,10 @@ int copy_streams(cudaStream_t* in, cudaStream_t* out) {
 }
 
 // ---- device error flag ---------------------------------------------------------
+ScheduleColumns::ScheduleColumns(i64 n) { t_schedule_columns = n; }
+ScheduleColumns::~ScheduleColumns() { t_schedule_columns = 0; }
+i64 schedule_columns(i64 n) { return t_schedule_columns ? t_schedule_columns : n; }
+
 int* device_error_flag() {
     std::lock_guard<std::mutex> lk(g_mu);
     DeviceCache& dc = g_cache[current_device()];

@@ -2042,7 +2042,7 @@ int launch_sk(const CUtensorMap* ma, const CUtensorMap* mb, Params* P, int nprod
 
 // Tiles of 128 x bn that the triangle mask keeps.
 inline i64 live_tiles(const Params& P, int bn) {
-    const i64 tn_all = cdiv(P.n, bn);
+    const i64 tn_all = cdiv(schedule_columns(P.n), bn);
     if (!P.tri) return i64(P.tiles_m) * tn_all;
     i64 live = 0;
     for (i64 tm = 0; tm < P.tiles_m; ++tm)

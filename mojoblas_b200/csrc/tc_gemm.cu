@@ -1883,7 +1883,7 @@ int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, Params& P, const cha
                                       C::SMEM_BYTES));
         mark_configured(configured, dev);
     }
-    P.err = device_error_flag();
+    if (!P.err) P.err = device_error_flag();
     const i64 tiles = i64(P.tiles_m) * P.tiles_n;
     if (tiles > 0x7fffffff) return MBG_ERR_UNSUPPORTED;
     ProfScope prof(name);
@@ -1933,7 +1933,7 @@ int ck_clusters(int dev, int S) {
 
 template <class C>
 int launch_ck(const CUtensorMap& ma, const CUtensorMap& mb, Params& P, int S, const char* name) {
-    P.err = device_error_flag();
+    if (!P.err) P.err = device_error_flag();
     const i64 ctas = i64(P.tiles_m) * P.tiles_n * S;
     if (ctas > 0x7fffffff) return MBG_ERR_UNSUPPORTED;
     ProfScope prof(name);
@@ -2017,7 +2017,7 @@ int launch_sk(const CUtensorMap* ma, const CUtensorMap* mb, Params* P, int nprod
     constexpr int R = C::TILE_M / BM;  // 128-row tiles per output tile
     i64 tiles[2] = {0, 0};
     for (int i = 0; i < nprod; ++i) {
-        P[i].err = device_error_flag();
+        if (!P[i].err) P[i].err = device_error_flag();
         tiles[i] = i64((P[i].tiles_m + R - 1) / R) * P[i].tiles_n;
         if (P[i].num_kb <= 0) return MBG_ERR_UNSUPPORTED;
         if (P[i].beta != 0.0 || P[i].tri || P[i].band != KB_NONE || P[i].dvec) stream_k = false;
@@ -2038,6 +2038,34 @@ int launch_sk(const CUtensorMap* ma, const CUtensorMap* mb, Params* P, int nprod
     split_sk_kernel<C><<<unsigned(G), C::THREADS, C::SMEM_BYTES, stream()>>>(ma[0], mb[0], P[0], ma[1], mb[1], P[1],
                                                                             W);
     return check_launch(name);
+}
+
+// Everything that launch_split_product may launch, loaded and configured ahead of its first use
+// (loading maps code on the device).
+template <class C>
+int prepare_split_kernel(int dev, int sms, bool wide) {
+    MBG_CUDA(cudaFuncSetAttribute(tc_gemm_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+    if (C::BN >= 128)
+        for (int S = 1; S <= CK_MAX; ++S) ck_clusters<C>(dev, S);
+    if (wide) {
+        i64 workers = 0;
+        MBG_CUDA(cudaFuncSetAttribute(split_sk_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+        MBG_TRY(sk_workers<C>(dev, sms, workers));
+        cudaFuncAttributes at;
+        MBG_CUDA(cudaFuncGetAttributes(&at, sk_zero_kernel<C>));
+    }
+    return MBG_OK;
+}
+int prepare_split_kernels() {
+    int dev = 0, sms = 148;
+    MBG_CUDA(cudaGetDevice(&dev));
+    MBG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    MBG_TRY(prepare_split_kernel<CfgBF16x3>(dev, sms, true));
+    MBG_TRY(prepare_split_kernel<CfgBF16x6>(dev, sms, true));
+    MBG_TRY(prepare_split_kernel<CfgBF16x3m>(dev, sms, false));
+    MBG_TRY(prepare_split_kernel<CfgBF16x6m>(dev, sms, false));
+    MBG_TRY(prepare_split_kernel<CfgBF16x3n>(dev, sms, false));
+    return prepare_split_kernel<CfgBF16x6n>(dev, sms, false);
 }
 
 // Tiles of 128 x bn that the triangle mask keeps.
@@ -2456,7 +2484,7 @@ int launch_ozaki(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap
         MBG_CUDA(cudaFuncSetAttribute(ozaki_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
         mark_configured(configured, dev);
     }
-    P.err = device_error_flag();
+    if (!P.err) P.err = device_error_flag();
     const i64 tiles = i64(P.tiles_m) * P.tiles_n;
     if (tiles > 0x7fffffff) return MBG_ERR_UNSUPPORTED;
     ProfScope prof("tc_gemm_ozaki");
@@ -2475,7 +2503,7 @@ int launch_ozaki_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtens
                                       C::SMEM_BYTES));
         mark_configured(configured, dev);
     }
-    P.err = device_error_flag();
+    if (!P.err) P.err = device_error_flag();
     i64 ctas = 2 * i64((P.tiles_m + 1) / 2) * P.tiles_n;
     if (ctas > 0x7fffffff) return MBG_ERR_UNSUPPORTED;
     if (tuning().ozaki_cta_pair == 2) {  // persistent: one cluster per pair of SMs
@@ -2668,10 +2696,7 @@ int noalloc_setup(NoallocDevice** out) {
         MBG_CUDA(cudaGetSymbolAddress(&p, g_noalloc_scratch));
         void* e = nullptr;
         MBG_CUDA(cudaGetSymbolAddress(&e, g_noalloc_err));
-        MBG_CUDA(cudaFuncSetAttribute(tc::tc_gemm_kernel<tc::CfgBF16x3>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, tc::CfgBF16x3::SMEM_BYTES));
-        MBG_CUDA(cudaFuncSetAttribute(tc::tc_gemm_kernel<tc::CfgBF16x6>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, tc::CfgBF16x6::SMEM_BYTES));
+        MBG_TRY(tc::prepare_split_kernels());
         d.scratch = p;
         d.err = static_cast<int*>(e);
         d.ready = true;
@@ -2745,20 +2770,12 @@ extern "C" int mbg_sgemm_ex_noalloc(int mode, char ta, char tb, int64_t m, int64
             noalloc_split<3>(b, ldb, is_n(tb), n, k, Np, Kp, pb);
         }
         MBG_TRY(check_launch("split_bf16"));
-        CUtensorMap ma, mb;
-        MBG_TRY(make_map(&ma, pa, false, Kp, Mp, terms, 64, BM));
-        MBG_TRY(make_map(&mb, pb, false, Kp, Np, terms, 64, 256));
         Params P{};
         P.m = m; P.n = n; P.num_kb = int(Kp / 32);
-        P.tiles_m = int(cdiv(m, BM)); P.tiles_n = int(cdiv(n, 256));
-        P.tri = 0; P.c = c; P.ldc = ldc; P.alpha = alpha; P.beta = beta;
+        P.tiles_m = int(cdiv(m, BM));
+        P.c = c; P.ldc = ldc; P.alpha = alpha; P.beta = beta;
         P.err = d->err;
-        const unsigned tiles = unsigned(i64(P.tiles_m) * P.tiles_n);
-        if (terms == 2)
-            tc_gemm_kernel<CfgBF16x3><<<tiles, CfgBF16x3::THREADS, CfgBF16x3::SMEM_BYTES, stream()>>>(ma, mb, P);
-        else
-            tc_gemm_kernel<CfgBF16x6><<<tiles, CfgBF16x6::THREADS, CfgBF16x6::SMEM_BYTES, stream()>>>(ma, mb, P);
-        MBG_TRY(check_launch(terms == 2 ? "tc_gemm_bf16x3" : "tc_gemm_bf16x6"));
+        MBG_TRY(launch_split_product(terms, pa, Mp, Mp, pb, Np, Kp, P));
     }
     // synchronous mode: wait, then report an expired wait (this entry point's flag is read
     // and cleared by read_and_clear_device_error, as mbg_synchronize does in asynchronous mode)

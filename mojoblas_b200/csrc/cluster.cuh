@@ -50,20 +50,22 @@ inline int usable_sms(int S) {
     return sms[S];
 }
 
-// A launch of `ctas` CTAs in clusters of S.
+// A launch of `ctas` CTAs in clusters of S; pdl: as launch_pdl.
 struct Launch {
     cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute attr{};
-    Launch(unsigned ctas, int S, int threads, size_t smem, cudaStream_t s) {
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = unsigned(S);
-        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchAttribute attr[2]{};
+    Launch(unsigned ctas, int S, int threads, size_t smem, cudaStream_t s, bool pdl = false) {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = unsigned(S);
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.gridDim = dim3(ctas);
         cfg.blockDim = dim3(unsigned(threads));
         cfg.dynamicSmemBytes = smem;
         cfg.stream = s;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = pdl ? 2 : 1;
     }
     Launch(const Launch&) = delete;
 };

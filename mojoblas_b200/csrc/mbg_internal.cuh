@@ -1,6 +1,8 @@
 // Internal declarations shared by the library's translation units.
 #pragma once
 
+#include <utility>
+
 #include <cuda_runtime.h>
 #include <atomic>
 #include <cstdint>
@@ -62,6 +64,29 @@ void set_error_msg(const std::string& msg);
 
 // Checks the launch that was just enqueued (configuration errors only).
 int check_launch(const char* name);
+
+// Launches that may start while the kernel before them on the stream still runs (programmatic
+// dependent launch).  Every kernel launched so calls pdl_wait() before its first access to
+// global memory: that returns once the kernel before has completed, and so, by induction, all
+// earlier work on the stream.  What comes before it (barriers, TMEM, descriptors) and the launch
+// itself then overlap the tail of the kernel before.  pdl_next() lets the next kernel start once
+// every block has called it.  Without the launch attribute both do nothing.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <class... P, class... A>
+inline cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
+}
 
 // A second non-blocking compute stream of the current device (created on first use,
 // kept), for independent work within one call that can run beside the library stream.

@@ -39,6 +39,7 @@
 // thread records an error code in the library's mapped error flag and the CTA
 // proceeds to teardown (TMEM is always freed).
 #include "mbg_internal.cuh"
+#include "cluster.cuh"
 #include "tc_ptx.cuh"
 
 #include <cuda.h>
@@ -212,34 +213,6 @@ __device__ __forceinline__ void split_store_row(const Params& P, const i64 row, 
     split_store<C::EPI_COLS>(Cm + row + cbase * P.ldc, P.ldc, alpha, float(P.beta), acc, lo, hi);
 }
 
-// ---- one tile's reduction over the CTAs of a cluster ----------------------------------------
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ uint32_t cluster_size() {
-    uint32_t r;
-    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t peer_smem(uint32_t addr, uint32_t rank) {
-    uint32_t r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ float4 peer_load4(uint32_t addr) {
-    float4 v;
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-                 : "r"(addr)
-                 : "memory");
-    return v;
-}
-
 // Output tile `tile` of the product P, its operands' planes read through tmA / tmB (kernel
 // parameters): one CTA's whole work in the kernels below.  CK: the CTAs of a cluster share the
 // tile, each taking an equal part of its slabs; then each leaves its sums in its own (by now
@@ -269,8 +242,12 @@ __device__ __forceinline__ void tc_gemm_tile(const CUtensorMap& tmA, const CUten
     if (P.band == KB_A_LOWER) tm = P.tiles_m - 1 - tm;
     if (P.band == KB_B_UPPER) tn = P.tiles_n - 1 - tn;
     const i64 m0 = i64(tm) * BM, n0 = i64(tn) * C::BN;
-    if (P.tri == 1 && m0 + BM <= n0) return;        // tile strictly above the diagonal
-    if (P.tri == 2 && m0 > n0 + C::BN - 1) return;  // tile strictly below the diagonal
+    pdl_next();
+    // tiles strictly above (below) the diagonal
+    if ((P.tri == 1 && m0 + BM <= n0) || (P.tri == 2 && m0 > n0 + C::BN - 1)) {
+        pdl_wait();
+        return;
+    }
 
     // slabs [kb0, kb0 + nkb) of the reduction: all of them, or the tile's band
     int kb0 = 0, nkb = P.num_kb;
@@ -281,7 +258,7 @@ __device__ __forceinline__ void tc_gemm_tile(const CUtensorMap& tmA, const CUten
         nkb = int(s1 - s0);
     }
     if constexpr (CK) {
-        const int S = int(cluster_size()), r = int(cluster_rank());
+        const int S = int(clu::size()), r = int(clu::rank());
         kb0 = nkb * r / S;
         nkb = nkb * (r + 1) / S - kb0;
     }
@@ -308,6 +285,7 @@ __device__ __forceinline__ void tc_gemm_tile(const CUtensorMap& tmA, const CUten
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -418,9 +396,9 @@ __device__ __forceinline__ void tc_gemm_tile(const CUtensorMap& tmA, const CUten
     if constexpr (CK) {
         static_assert(BM * C::BN * 4 <= C::STAGES * C::STAGE_BYTES, "the sums reuse the stage buffers");
         __syncwarp();
-        cluster_sync_all();
+        clu::sync_all();
         if (warp >= 2) {
-            const int S = int(cluster_size()), r = int(cluster_rank());
+            const int S = int(clu::size()), r = int(clu::rank());
             constexpr int UNITS = C::BN / 16;
             const int c0 = 16 * (UNITS * r / S), c1 = 16 * (UNITS * (r + 1) / S);  // this CTA's columns of the tile
             const int quarter = warp & 3, part = (warp - 2) >> 2;
@@ -436,9 +414,9 @@ __device__ __forceinline__ void tc_gemm_tile(const CUtensorMap& tmA, const CUten
 #pragma unroll
                     for (int u = 0; u < 4; ++u)
                         if (s0 + u < S) {
-                            const uint32_t q = peer_smem(base, uint32_t(s0 + u)) + uint32_t(c / 4 * BM * 16);
+                            const uint32_t q = clu::peer(base, uint32_t(s0 + u)) + uint32_t(c / 4 * BM * 16);
 #pragma unroll
-                            for (int j = 0; j < 4; ++j) t[u][j] = peer_load4(q + uint32_t(j * BM * 16));
+                            for (int j = 0; j < 4; ++j) t[u][j] = clu::load4(q + uint32_t(j * BM * 16));
                         }
 #pragma unroll
                     for (int u = 0; u < 4; ++u)
@@ -458,7 +436,7 @@ __device__ __forceinline__ void tc_gemm_tile(const CUtensorMap& tmA, const CUten
             }
         }
         __syncwarp();
-        cluster_sync_all();  // no CTA leaves while another reads its sums
+        clu::sync_all();  // no CTA leaves while another reads its sums
     }
 }
 
@@ -475,7 +453,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 template <class C>
 __global__ void __launch_bounds__(C::THREADS, 1)
 tc_gemm_ck_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Params P) {
-    tc_gemm_tile<C, true>(tmA, tmB, P, int(blockIdx.x / cluster_size()));
+    tc_gemm_tile<C, true>(tmA, tmB, P, int(blockIdx.x / clu::size()));
 }
 
 // ---------------------------------------------------------------------------
@@ -789,8 +767,12 @@ ozaki_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     if (P.band == KB_A_LOWER) tm = P.tiles_m - 1 - tm;
     if (P.band == KB_B_UPPER) tn = P.tiles_n - 1 - tn;
     const i64 m0 = i64(tm) * BM, n0 = i64(tn) * C::BN;
-    if (P.tri == 1 && m0 + BM <= n0) return;        // tile strictly above the diagonal
-    if (P.tri == 2 && m0 > n0 + C::BN - 1) return;  // tile strictly below the diagonal
+    pdl_next();
+    // tiles strictly above (below) the diagonal
+    if ((P.tri == 1 && m0 + BM <= n0) || (P.tri == 2 && m0 > n0 + C::BN - 1)) {
+        pdl_wait();
+        return;
+    }
 
     // slabs [kb0, kb0 + nkb) of the reduction: all of them, or the tile's band
     int kb0 = 0, nkb = P.num_kb;
@@ -1093,7 +1075,8 @@ ozaki_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     uint64_t* tempty = tfull + 1;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 1);
 
-    const uint32_t rank = cluster_rank();  // 0: leader (issues the MMAs), 1: peer
+    pdl_next();
+    const uint32_t rank = clu::rank();  // 0: leader (issues the MMAs), 1: peer
     const int ntiles = ((P.tiles_m + 1) >> 1) * P.tiles_n;
     const int first = blockIdx.x >> 1, stride = gridDim.x >> 1;
 
@@ -1112,10 +1095,11 @@ ozaki_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         tmem_relinquish_pair();
     }
     tc_fence_before();
-    cluster_sync_all();  // barriers of both CTAs initialised, TMEM of the pair allocated
+    clu::sync_all();  // barriers of both CTAs initialised, TMEM of the pair allocated
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     const uint32_t leader_tempty = peer_addr(tempty, 0);
+    pdl_wait();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -1207,7 +1191,7 @@ ozaki_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
     tc_fence_before();
     __syncwarp();
-    cluster_sync_all();  // the peer's epilogue and loads are done; no more remote barrier traffic
+    clu::sync_all();  // the peer's epilogue and loads are done; no more remote barrier traffic
     if (warp == 0) {
         __syncwarp();
         tc_fence_after();
@@ -1314,6 +1298,8 @@ __device__ __forceinline__ bool sk_next(const SkWork& W, const Params& P0, const
 // a tile long, so each such tile holds one boundary).
 template <class C>
 __global__ void __launch_bounds__(256) sk_zero_kernel(Params P0, Params P1, SkWork W, int workers) {
+    pdl_next();
+    pdl_wait();
     const i64 n = W.total - W.sk_begin;
     const i64 pos = W.sk_begin + (i64(blockIdx.x) + 1) * n / workers;
     int prod, tile, kb, nkb;
@@ -1358,6 +1344,7 @@ split_sk_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant_
     uint64_t* tempty = tfull + 2;         // [2]: epilogue finished reading a buffer
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
     int* const err = P0.err;
+    pdl_next();
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -1379,6 +1366,7 @@ split_sk_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -1563,6 +1551,8 @@ template <int TERMS, bool KMAJOR>
 __global__ void __launch_bounds__(256)
 split_bf16_kernel(const float* __restrict__ src, i64 ld, i64 rows, i64 K, i64 Rp, i64 Kp,
                   __nv_bfloat16* __restrict__ planes, int keep = 0) {
+    pdl_next();
+    pdl_wait();
     const i64 r0 = i64(blockIdx.y) * SP_R, l0 = i64(blockIdx.x) * SP_K;
     const size_t plane = size_t(Rp) * size_t(Kp);
     const bool vec = reinterpret_cast<uintptr_t>(src) % 16 == 0 && ld % 4 == 0 && keep == 0;
@@ -1624,6 +1614,8 @@ template <int TERMS>
 __global__ void __launch_bounds__(256)
 split_bf16_both_kernel(const float* __restrict__ src, i64 ld, i64 gm, i64 gn, __nv_bfloat16* __restrict__ pr,
                        i64 RpR, i64 KpR, __nv_bfloat16* __restrict__ pc, i64 RpC, i64 KpC) {
+    pdl_next();
+    pdl_wait();
     const i64 i0 = i64(blockIdx.y) * SP_R, j0 = i64(blockIdx.x) * SP_K;  // rows i of G, columns j
     const bool vec = reinterpret_cast<uintptr_t>(src) % 16 == 0 && ld % 4 == 0;
     __shared__ float tile[SP_K][SP_R + 1];  // tile[j][i]
@@ -1682,6 +1674,8 @@ __device__ __forceinline__ void oz_exponent_max(int* e, i64 r, double mx) {
 template <bool KMAJOR>
 __global__ void __launch_bounds__(256)
 row_exponent_kernel(const double* __restrict__ src, i64 ld, i64 rows, i64 K, int* __restrict__ e, int keep) {
+    pdl_next();
+    pdl_wait();
     if (KMAJOR) {  // warp per row and k chunk, lanes along k (coalesced)
         const i64 r = i64(blockIdx.x) * 8 + (threadIdx.x >> 5);
         if (r >= rows) return;
@@ -1763,6 +1757,8 @@ template <bool KMAJOR>
 __global__ void __launch_bounds__(256)
 slice_i8_kernel(const double* __restrict__ src, i64 ld, i64 rows, i64 K, i64 Rp, i64 Kp, int slices,
                 int* __restrict__ e, int8_t* __restrict__ planes, int keep) {
+    pdl_next();
+    pdl_wait();
     __shared__ double tile[PT_R][PT_K + 1];
     const i64 r0 = i64(blockIdx.y) * PT_R, l0 = i64(blockIdx.x) * PT_K;
     load_tile<double, KMAJOR>(src, ld, rows, K, r0, l0, keep, tile);
@@ -1887,38 +1883,20 @@ int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, Params& P, const cha
     const i64 tiles = i64(P.tiles_m) * P.tiles_n;
     if (tiles > 0x7fffffff) return MBG_ERR_UNSUPPORTED;
     ProfScope prof(name);
-    tc_gemm_kernel<C><<<unsigned(tiles), C::THREADS, C::SMEM_BYTES, stream()>>>(ma, mb, P);
+    MBG_CUDA(launch_pdl(tc_gemm_kernel<C>, dim3(unsigned(tiles)), dim3(C::THREADS), C::SMEM_BYTES, stream(), ma, mb, P));
     return check_launch(name);
 }
-
-// Launch attributes of tc_gemm_ck_kernel with S CTAs per cluster.
-struct CkLaunch {
-    cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute attr{};
-    CkLaunch(unsigned ctas, int S, int threads, int smem, cudaStream_t s) {
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = unsigned(S);
-        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-        cfg.gridDim = dim3(ctas);
-        cfg.blockDim = dim3(unsigned(threads));
-        cfg.dynamicSmemBytes = size_t(smem);
-        cfg.stream = s;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-    }
-};
-constexpr int CK_MAX = 8;  // CTAs per cluster (portable)
 
 // Clusters of S CTAs of tc_gemm_ck_kernel<C> that can be resident at once (0: none), cached
 // per device.
 template <class C>
 int ck_clusters(int dev, int S) {
-    static std::atomic<int> cache[64][CK_MAX + 1];  // count + 1
+    static std::atomic<int> cache[64][clu::MAX_CTAS + 1];  // count + 1
     if (dev < 0 || dev >= 64) return 0;
     int v = cache[dev][S].load();
     if (!v) {
         int n = 0;
-        const CkLaunch l(unsigned(S), S, C::THREADS, C::SMEM_BYTES, nullptr);
+        const clu::Launch l(unsigned(S), S, C::THREADS, C::SMEM_BYTES, nullptr);
         if (cudaFuncSetAttribute(tc_gemm_ck_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES) !=
                 cudaSuccess ||
             cudaOccupancyMaxActiveClusters(&n, tc_gemm_ck_kernel<C>, &l.cfg) != cudaSuccess) {
@@ -1937,7 +1915,7 @@ int launch_ck(const CUtensorMap& ma, const CUtensorMap& mb, Params& P, int S, co
     const i64 ctas = i64(P.tiles_m) * P.tiles_n * S;
     if (ctas > 0x7fffffff) return MBG_ERR_UNSUPPORTED;
     ProfScope prof(name);
-    const CkLaunch l(unsigned(ctas), S, C::THREADS, C::SMEM_BYTES, stream());
+    const clu::Launch l(unsigned(ctas), S, C::THREADS, C::SMEM_BYTES, stream(), true);
     MBG_CUDA(cudaLaunchKernelEx(&l.cfg, tc_gemm_ck_kernel<C>, ma, mb, P));
     return check_launch(name);
 }
@@ -2032,11 +2010,11 @@ int launch_sk(const CUtensorMap* ma, const CUtensorMap* mb, Params* P, int nprod
     if (G <= 0) return MBG_OK;
     ProfScope prof(name);
     if (W.total > W.sk_begin && G > 1) {
-        sk_zero_kernel<C><<<unsigned(G - 1), 256, 0, stream()>>>(P[0], P[1], W, int(G));
+        MBG_CUDA(launch_pdl(sk_zero_kernel<C>, dim3(unsigned(G - 1)), dim3(256), 0, stream(), P[0], P[1], W, int(G)));
         MBG_TRY(check_launch("sk_zero"));
     }
-    split_sk_kernel<C><<<unsigned(G), C::THREADS, C::SMEM_BYTES, stream()>>>(ma[0], mb[0], P[0], ma[1], mb[1], P[1],
-                                                                            W);
+    MBG_CUDA(launch_pdl(split_sk_kernel<C>, dim3(unsigned(G)), dim3(C::THREADS), C::SMEM_BYTES, stream(), ma[0], mb[0], P[0],
+                        ma[1], mb[1], P[1], W));
     return check_launch(name);
 }
 
@@ -2046,7 +2024,7 @@ template <class C>
 int prepare_split_kernel(int dev, int sms, bool wide) {
     MBG_CUDA(cudaFuncSetAttribute(tc_gemm_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
     if (C::BN >= 128)
-        for (int S = 1; S <= CK_MAX; ++S) ck_clusters<C>(dev, S);
+        for (int S = 1; S <= clu::MAX_CTAS; ++S) ck_clusters<C>(dev, S);
     if (wide) {
         i64 workers = 0;
         MBG_CUDA(cudaFuncSetAttribute(split_sk_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
@@ -2100,7 +2078,7 @@ SplitShape split_shape(const Params& P, int terms, int dev, int sms) {
     double t_best = 0;
     for (int bn = 256; bn >= 64; bn /= 2) {
         const i64 tiles = imax(1, live_tiles(P, bn));
-        for (int S = 1; S <= (bn >= 128 && P.band == KB_NONE && !P.dvec ? CK_MAX : 1) && S <= P.num_kb; ++S) {
+        for (int S = 1; S <= (bn >= 128 && P.band == KB_NONE && !P.dvec ? clu::MAX_CTAS : 1) && S <= P.num_kb; ++S) {
             const i64 room = S == 1 ? sms : bn == 256 ? ck_clusters<Wide>(dev, S) : ck_clusters<Mid>(dev, S);
             if (room <= 0) continue;
             const double busy = double(imin(tiles, room) * S) / sms;
@@ -2163,8 +2141,8 @@ int launch_split(const float* src, i64 ld, bool kmajor, i64 rows, i64 K, i64 Rp,
     ProfScope prof("split_bf16");
     const dim3 g = split_grid(Rp, Kp);
     if (Rp / SP_R > 65535) return MBG_ERR_UNSUPPORTED;
-    if (kmajor) split_bf16_kernel<TERMS, true><<<g, 256, 0, stream()>>>(src, ld, rows, K, Rp, Kp, planes, keep);
-    else split_bf16_kernel<TERMS, false><<<g, 256, 0, stream()>>>(src, ld, rows, K, Rp, Kp, planes, keep);
+    MBG_CUDA(launch_pdl(kmajor ? split_bf16_kernel<TERMS, true> : split_bf16_kernel<TERMS, false>, g, dim3(256), 0,
+                        stream(), src, ld, rows, K, Rp, Kp, planes, keep));
     return check_launch("split_bf16");
 }
 
@@ -2181,6 +2159,8 @@ template <bool SCALE>
 __global__ void __launch_bounds__(256)
 slice_rows_kmajor_kernel(const double* src, i64 ld, i64 rows, i64 K, i64 Rp, i64 Kp, int slices,
                          int* __restrict__ e, int8_t* __restrict__ planes, int keep, const double* __restrict__ dscale) {
+    pdl_next();
+    pdl_wait();
     const i64 r = i64(blockIdx.x) * 8 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (r >= Rp) return;
@@ -2262,11 +2242,11 @@ int launch_slices(const double* src, i64 ld, bool kmajor, i64 rows, i64 K, i64 R
         ProfScope prof("ozaki_slice");
         const unsigned g = unsigned(cdiv(Rp, 8));
         if (dscale)
-            slice_rows_kmajor_kernel<true><<<g, 256, 0, stream()>>>(src, ld, rows, K, Rp, Kp, slices, e, planes, keep,
-                                                                  dscale);
+            MBG_CUDA(launch_pdl(slice_rows_kmajor_kernel<true>, g, dim3(256), 0, stream(), src, ld, rows, K, Rp, Kp, slices, e, planes, keep,
+                                                                  dscale));
         else
-            slice_rows_kmajor_kernel<false><<<g, 256, 0, stream()>>>(src, ld, rows, K, Rp, Kp, slices, e, planes,
-                                                                   keep, nullptr);
+            MBG_CUDA(launch_pdl(slice_rows_kmajor_kernel<false>, g, dim3(256), 0, stream(), src, ld, rows, K, Rp, Kp, slices, e, planes,
+                                                                   keep, nullptr));
         return check_launch("ozaki_slice");
     }
     {
@@ -2275,19 +2255,19 @@ int launch_slices(const double* src, i64 ld, bool kmajor, i64 rows, i64 K, i64 R
         if (kmajor) {
             dim3 g(unsigned(cdiv(rows, 8)), unsigned(cdiv(K, OZ_EXP_KWARP)));
             if (g.y > 65535) return MBG_ERR_UNSUPPORTED;
-            row_exponent_kernel<true><<<g, 256, 0, stream()>>>(src, ld, rows, K, e, keep);
+            MBG_CUDA(launch_pdl(row_exponent_kernel<true>, g, dim3(256), 0, stream(), src, ld, rows, K, e, keep));
         } else {
             dim3 g(unsigned(cdiv(rows, 32)), unsigned(cdiv(K, OZ_EXP_KCHUNK)));
             if (g.y > 65535) return MBG_ERR_UNSUPPORTED;
-            row_exponent_kernel<false><<<g, 256, 0, stream()>>>(src, ld, rows, K, e, keep);
+            MBG_CUDA(launch_pdl(row_exponent_kernel<false>, g, dim3(256), 0, stream(), src, ld, rows, K, e, keep));
         }
         MBG_TRY(check_launch("ozaki_exponent"));
     }
     ProfScope prof("ozaki_slice");
     dim3 g(unsigned(Kp / PT_K), unsigned(Rp / PT_R));
     if (g.y > 65535) return MBG_ERR_UNSUPPORTED;
-    if (kmajor) slice_i8_kernel<true><<<g, 256, 0, stream()>>>(src, ld, rows, K, Rp, Kp, slices, e, planes, keep);
-    else slice_i8_kernel<false><<<g, 256, 0, stream()>>>(src, ld, rows, K, Rp, Kp, slices, e, planes, keep);
+    MBG_CUDA(launch_pdl(kmajor ? slice_i8_kernel<true> : slice_i8_kernel<false>, g, dim3(256), 0, stream(), src, ld, rows, K,
+                        Rp, Kp, slices, e, planes, keep));
     return check_launch("ozaki_slice");
 }
 
@@ -2435,12 +2415,8 @@ int sgemm_split_tc_dual(int terms, const SplitProduct& x, const SplitProduct& y)
             if (gi / SP_R > 65535) continue;
             const dim3 g(unsigned(gj / SP_K), unsigned(gi / SP_R));
             ProfScope prof("split_bf16");
-            if (terms == 2)
-                split_bf16_both_kernel<2><<<g, 256, 0, stream()>>>(r.src, r.ld, r.rows, r.K, r.planes, r.Rp, r.Kp,
-                                                                   c.planes, c.Rp, c.Kp);
-            else
-                split_bf16_both_kernel<3><<<g, 256, 0, stream()>>>(r.src, r.ld, r.rows, r.K, r.planes, r.Rp, r.Kp,
-                                                                   c.planes, c.Rp, c.Kp);
+            MBG_CUDA(launch_pdl(terms == 2 ? split_bf16_both_kernel<2> : split_bf16_both_kernel<3>, g, dim3(256), 0,
+                                stream(), r.src, r.ld, r.rows, r.K, r.planes, r.Rp, r.Kp, c.planes, c.Rp, c.Kp));
             MBG_TRY(check_launch("split_bf16"));
             a.done = b.done = true;
         }
@@ -2512,7 +2488,7 @@ int launch_ozaki_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtens
         ctas = imin(ctas, i64(sms / 2) * 2);
     }
     ProfScope prof("tc_gemm_ozaki");
-    ozaki_pair_kernel<C><<<unsigned(ctas), C::THREADS, C::SMEM_BYTES, stream()>>>(ma, mb, mal, mbl, P);
+    MBG_CUDA(launch_pdl(ozaki_pair_kernel<C>, dim3(unsigned(ctas)), dim3(C::THREADS), C::SMEM_BYTES, stream(), ma, mb, mal, mbl, P));
     return check_launch("tc_gemm_ozaki");
 }
 

@@ -405,6 +405,8 @@ template <typename T, bool LOWER, bool TRANS, bool UNIT>
 __global__ void __launch_bounds__(BS_THREADS, 1)
 block_invert_kernel(i64 m, int nbi, const T* __restrict__ A, i64 lda, T* __restrict__ W, i64 ldw) {
     extern __shared__ __align__(16) unsigned char bs_smem_raw[];
+    pdl_next();
+    pdl_wait();
     const i64 r0 = i64(blockIdx.y) * nbi;
     const int nbb = int(min(i64(nbi), m - r0));
     const i64 c0 = i64(blockIdx.x) * BS_COLS;
@@ -427,6 +429,8 @@ block_invert_f32_kernel(i64 m, int nbi, const float* __restrict__ A, i64 lda, bo
                         float* __restrict__ W, i64 ldw, int* err) {
     extern __shared__ __align__(16) float inv_smem[];
     __shared__ uint64_t bars[INV_MAXBLK];
+    pdl_next();
+    pdl_wait();
     const i64 r0 = i64(blockIdx.y) * nbi;
     const int nbb = int(min(i64(nbi), m - r0)), c0 = int(blockIdx.x) * ws::RB;
     if (c0 >= nbb) return;
@@ -471,7 +475,7 @@ int launch_block_invert_t(i64 m, int nbi, const T* a, i64 lda, T* w, i64 ldw) {
         mark_configured(configured, dev);
     }
     const dim3 g(unsigned(cdiv(nbi, BS_COLS)), unsigned(cdiv(m, nbi)));
-    kern<<<g, BS_THREADS, bs_smem_bytes<T>(nbi), stream()>>>(m, nbi, a, lda, w, ldw);
+    MBG_CUDA(launch_pdl(kern, g, dim3(BS_THREADS), bs_smem_bytes<T>(nbi), stream(), m, nbi, a, lda, w, ldw));
     return check_launch("trsm_block_invert");
 }
 
@@ -486,8 +490,8 @@ int launch_block_invert_f32(bool lower, bool trans, bool unit, i64 m, int nbi, c
         mark_configured(configured, dev);
     }
     const dim3 g(unsigned(cdiv(nbi, ws::RB)), unsigned(cdiv(m, nbi)));
-    block_invert_f32_kernel<<<g, 32 * INV_WARPS, INV_SMEM, stream()>>>(m, nbi, a, lda, lower, trans, unit, w, ldw,
-                                                                       device_error_flag());
+    MBG_CUDA(launch_pdl(block_invert_f32_kernel, g, dim3(32 * INV_WARPS), INV_SMEM, stream(), m, nbi, a, lda, lower, trans,
+                        unit, w, ldw, device_error_flag()));
     return check_launch("trsm_block_invert");
 }
 
@@ -537,6 +541,8 @@ template <> struct InvPlanes<float> {
 // thread that overwrites it.
 __global__ void split_block_diagonal_kernel(i64 m, int nbi, double* __restrict__ W, i64 ldw,
                                             double* __restrict__ d) {
+    pdl_next();
+    pdl_wait();
     for (i64 r = blockIdx.x * (i64)blockDim.x + threadIdx.x; r < m; r += (i64)gridDim.x * blockDim.x) {
         double* p = W + r + (r % nbi) * ldw;
         d[r] = *p;
@@ -550,7 +556,8 @@ template <> struct InvPlanes<double> {
     int make(int, int slices, i64 m, i64 nbi, double* w) {
         MBG_TRY(wd.reserve(sizeof(double) * size_t(m)));
         d = wd.as<double>();
-        split_block_diagonal_kernel<<<unsigned(imin(cdiv(m, 256), 1024)), 256, 0, stream()>>>(m, int(nbi), w, m, d);
+        MBG_CUDA(launch_pdl(split_block_diagonal_kernel, dim3(unsigned(imin(cdiv(m, 256), 1024))), dim3(256), 0, stream(), m,
+                            int(nbi), w, m, d));
         MBG_TRY(check_launch("trsm_block_invert"));
         return ozaki_slice_a(slices, 'N', m, nbi, w, m, p);
     }

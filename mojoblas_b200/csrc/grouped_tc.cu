@@ -360,7 +360,7 @@ grouped_tc_kernel(const TcDesc* __restrict__ probs, const TcTile* __restrict__ t
                             const uint32_t accumulate = (kin > 0 || ks > 0 || pi > 0) ? 1u : 0u;
                             const uint64_t ad = smem_desc(sa + p * C::A_PLANE + ks * 32, 8 * GBKB, 4);
                             const uint64_t bd = smem_desc(sb + q * C::B_PLANE + ks * 32, 8 * GBKB, 4);
-                            umma<false>(tmem + uint32_t(buf * GBN), ad, bd, idesc, accumulate);
+                            umma<false>(tmem + uint32_t(buf * GBN), ad, bd, idesc, accumulate, collector);
                         }
                     }
                     umma_commit(&empty[s]);

@@ -1431,7 +1431,7 @@ split_sk_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant_
                             const uint32_t accumulate = (kin > 0 || ks > 0 || pi > 0) ? 1u : 0u;
                             const uint64_t ad = smem_desc(sa + p * C::A_PLANE + ks * 32, C::SBO, C::LAYOUT);
                             const uint64_t bd = smem_desc(sb + q * C::B_PLANE + ks * 32, C::SBO, C::LAYOUT);
-                            umma<false>(tmem + uint32_t(buf * C::BN), ad, bd, C::IDESC, accumulate);
+                            umma<false>(tmem + uint32_t(buf * C::BN), ad, bd, C::IDESC, accumulate, collector);
                         }
                     }
                     umma_commit(&empty[s]);  // slot s is free once these MMAs have read it
@@ -2875,7 +2875,7 @@ __global__ void __launch_bounds__(128, 1) mma_probe_kernel(int iters, int* err) 
         const uint64_t ad = smem_desc(sa, 1024, 2), bd = smem_desc(sb, 1024, 2);
         const uint32_t idesc = instr_desc(INT8, 128, 256);
 #pragma unroll 1
-        for (int i = 0; i < iters; ++i) umma<INT8>(tmem, ad, bd, idesc, i > 0 ? 1u : 0u);
+        for (int i = 0; i < iters; ++i) umma<INT8>(tmem, ad, bd, idesc, i > 0 ? 1u : 0u, 0);
         umma_commit(done);
         mbar_wait(done, 0, err, 98);
     }

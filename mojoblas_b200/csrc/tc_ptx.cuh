@@ -109,14 +109,17 @@ __device__ __forceinline__ void tc_fence_after() {
                  : "memory")
 template <bool INT8>
 __device__ __forceinline__ void umma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                     uint32_t accumulate, int collector = 0) {
+                                     uint32_t accumulate, int collector) {
     if (INT8) {
         if (collector == 1) MBG_UMMA("i8", ".collector::a::fill");
         else if (collector == 2) MBG_UMMA("i8", ".collector::a::use");
         else if (collector == 3) MBG_UMMA("i8", ".collector::a::lastuse");
         else MBG_UMMA("i8", "");
     } else {
-        MBG_UMMA("f16", "");
+        if (collector == 1) MBG_UMMA("f16", ".collector::a::fill");
+        else if (collector == 2) MBG_UMMA("f16", ".collector::a::use");
+        else if (collector == 3) MBG_UMMA("f16", ".collector::a::lastuse");
+        else MBG_UMMA("f16", "");
     }
 }
 #undef MBG_UMMA
@@ -172,12 +175,13 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// Product table, index -> (p, q) and collector use.
-//   split: ordered by descending p+q so small contributions enter the fp32
-//          accumulator first;
-//   ozaki: ordered by p (A slice), q ascending, so the products that share A_p
-//          run back to back and reuse it from the collector buffer; the first
-//          product into diagonal d is then (0, d).
+// Product table, index -> (p, q) and collector use: the products that share A_p run back to
+// back, the first filling the collector buffer and the others taking A_p from it.
+//   split: p and q descending, so that small contributions tend to enter the fp32 accumulator
+//          first.  A 128-column product reads 4 KB of A and 4 KB of B per 64 cycles, all that
+//          shared memory delivers; A from the collector in three of six products leaves room for the
+//          writes (8192^3 NT in six products, at the power limit: 4.83 -> 4.74 ms);
+//   ozaki: p and q ascending, so the first product into diagonal d is (0, d).
 template <int TERMS, bool OZAKI>
 __device__ __forceinline__ void product(int idx, int& p, int& q, int& collector) {
     collector = 0;
@@ -197,11 +201,15 @@ __device__ __forceinline__ void product(int idx, int& p, int& q, int& collector)
         return;
     }
     int t = 0;
-    for (int d = TERMS - 1; d >= 0; --d) {
-        for (int pp = 0; pp <= d; ++pp) {
-            if (t == idx) { p = pp; q = d - pp; return; }
-            ++t;
+    for (int pp = TERMS - 1; pp >= 0; --pp) {
+        const int cnt = TERMS - pp;  // q = cnt - 1 .. 0
+        if (idx < t + cnt) {
+            p = pp;
+            q = cnt - 1 - (idx - t);
+            if (cnt > 1) collector = (idx == t) ? 1 : (q == 0 ? 3 : 2);
+            return;
         }
+        t += cnt;
     }
     p = q = 0;
 }

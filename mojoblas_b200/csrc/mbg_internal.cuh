@@ -227,7 +227,6 @@ struct GroupedTcPlan {
     int terms = 3;
     void* table = nullptr;
     int count = 0, ntiles = 0, grid = 0;
-    size_t tiles_off = 0;
     int* err = nullptr;  // the library's wait-error flag, created before the graph capture
 };
 int grouped_tc_build(int terms, int count, const mbg_sgemm_problem* probs, GroupedTcPlan& out);

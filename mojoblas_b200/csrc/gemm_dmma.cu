@@ -83,6 +83,8 @@ __global__ void __launch_bounds__(C::THREADS, 1)
 gemm_dmma_kernel(i64 m, i64 n, i64 k, double alpha, const double* __restrict__ A, i64 lda,
                  const double* __restrict__ B, i64 ldb, double beta, double* __restrict__ Cm, i64 ldc, int band) {
     extern __shared__ __align__(16) double dsm[];
+    pdl_next();
+    pdl_wait();
     // A: TA (k contiguous in memory) -> [m][DKP], else [k][BM + 8]; B: !TB -> [n][DKP], else [k][BN + 8]
     constexpr int LA = TA ? DKP : BM + 8, LB = TB ? BN + 8 : DKP;
     double* As = dsm;
@@ -277,8 +279,9 @@ int launch_dmma_v(bool ta, bool tb, dim3 grid, i64 m, i64 n, i64 k, double alpha
         mark_configured(configured, dev);
     }
     cudaStream_t s = stream();
-#define DM(TA_, TB_) \
-    gemm_dmma_kernel<C, TA_, TB_, TRI, BM, BN, VEC><<<grid, C::THREADS, C::SMEM, s>>>(m, n, k, alpha, a, lda, b, ldb, beta, c, ldc, band)
+#define DM(TA_, TB_)                                                                                                \
+    MBG_CUDA(launch_pdl(gemm_dmma_kernel<C, TA_, TB_, TRI, BM, BN, VEC>, grid, dim3(C::THREADS), C::SMEM, s, m, n, k, \
+                        alpha, a, lda, b, ldb, beta, c, ldc, band))
     if (!ta && !tb) DM(false, false);
     else if (!ta && tb) DM(false, true);
     else if (ta && !tb) DM(true, false);
@@ -307,7 +310,7 @@ int launch_dmma_ck_t(int S, i64 m, i64 n, i64 k, double alpha, const double* a, 
         MBG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Small::SMEM));
         mark_configured(configured, dev);
     }
-    clu::Launch l(unsigned(cdiv(m, 64)) * unsigned(S), S, Small::THREADS, Small::SMEM, stream());
+    clu::Launch l(unsigned(cdiv(m, 64)) * unsigned(S), S, Small::THREADS, Small::SMEM, stream(), true);
     l.cfg.gridDim.y = unsigned(cdiv(n, 64));
     MBG_CUDA(cudaLaunchKernelEx(&l.cfg, kern, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc, int(KB_NONE)));
     return check_launch("gemm_dmma_f64");

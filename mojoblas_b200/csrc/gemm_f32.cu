@@ -21,6 +21,8 @@ __global__ void __launch_bounds__(FNT, FT == 128 ? 2 : 4)
 gemm_f32_kernel(i64 m, i64 n, i64 k, float alpha, const float* __restrict__ A, i64 lda,
                 const float* __restrict__ B, i64 ldb, float beta, float* __restrict__ C, i64 ldc, int band) {
     extern __shared__ __align__(16) float fsm[];
+    pdl_next();
+    pdl_wait();
     i64 tm, tn;
     if (TRI == 0) {
         tm = blockIdx.x;
@@ -42,6 +44,8 @@ __global__ void __launch_bounds__(FNT, FT == 128 ? 2 : 4)
 gemm_f32_ck_kernel(i64 m, i64 n, i64 k, float alpha, const float* __restrict__ A, i64 lda,
                    const float* __restrict__ B, i64 ldb, float beta, float* __restrict__ C, i64 ldc, unsigned tiles_m) {
     extern __shared__ __align__(16) float fsm[];
+    pdl_next();
+    pdl_wait();
     const unsigned tile = blockIdx.x / clu::size();
     f32_tile<FT, TA, TB, 0, VA, VB, true>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tile % tiles_m, tile / tiles_m,
                                           fsm);
@@ -60,7 +64,7 @@ int launch_f32_ck_t(int S, i64 m, i64 n, i64 k, float alpha, const float* a, i64
         mark_configured(configured, dev);
     }
     const unsigned gm = unsigned(cdiv(m, FT));
-    const clu::Launch l(gm * unsigned(cdiv(n, FT)) * unsigned(S), S, FNT, SM, stream());
+    const clu::Launch l(gm * unsigned(cdiv(n, FT)) * unsigned(S), S, FNT, SM, stream(), true);
     MBG_CUDA(cudaLaunchKernelEx(&l.cfg, gemm_f32_ck_kernel<FT, TA, TB, VA, VB>, m, n, k, alpha, a, lda, b, ldb, beta,
                                 c, ldc, gm));
     return check_launch("gemm_f32");
@@ -141,8 +145,9 @@ int launch_f32_v(bool ta, bool tb, dim3 grid, i64 m, i64 n, i64 k, float alpha, 
         mark_configured(configured, dev);
     }
     cudaStream_t s = stream();
-#define F32(TA_, TB_) \
-    gemm_f32_kernel<FT, TA_, TB_, TRI, VA, VB><<<grid, FNT, SM, s>>>(m, n, k, alpha, a, lda, b, ldb, beta, c, ldc, band)
+#define F32(TA_, TB_)                                                                                             \
+    MBG_CUDA(launch_pdl(gemm_f32_kernel<FT, TA_, TB_, TRI, VA, VB>, grid, dim3(FNT), SM, s, m, n, k, alpha, a, lda, b, \
+                        ldb, beta, c, ldc, band))
     if (!ta && !tb) F32(false, false);
     else if (!ta && tb) F32(false, true);
     else if (ta && !tb) F32(true, false);

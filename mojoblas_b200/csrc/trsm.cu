@@ -29,6 +29,7 @@
 // triangle is nonzero.
 #include "mbg_internal.cuh"
 #include "block_solve.cuh"
+#include "warp_invert_f64.cuh"
 #include "warp_solve.cuh"
 
 #include <vector>
@@ -399,31 +400,52 @@ int launch_copy(i64 m, i64 n, T alpha, const T* x, i64 ldx, T* y, i64 ldy) {
 // the substitution's by cond(A_bb) times the working precision (triangular inverses,
 // Higham, Accuracy and Stability of Numerical Algorithms, ch. 8 and 14).
 
-// W (m x NBI, column-major, ldw) block b := inv(op(A)_bb), solved against identity columns
-// made in shared memory: blockIdx.y = b, blockIdx.x = 32-column strip of the block.
-template <typename T, bool LOWER, bool TRANS, bool UNIT>
-__global__ void __launch_bounds__(BS_THREADS, 1)
-block_invert_kernel(i64 m, int nbi, const T* __restrict__ A, i64 lda, T* __restrict__ W, i64 ldw) {
-    extern __shared__ __align__(16) unsigned char bs_smem_raw[];
-    pdl_next();
-    pdl_wait();
-    const i64 r0 = i64(blockIdx.y) * nbi;
-    const int nbb = int(min(i64(nbi), m - r0));
-    const i64 c0 = i64(blockIdx.x) * BS_COLS;
-    if (c0 >= nbb) return;
-    bs::block_solve_strip<T, LOWER, TRANS, UNIT, BS_COLS, true>(nbb, nbb, A + r0 + r0 * lda, lda, W + r0, ldw, c0,
-                                                                   T(1), bs_smem_raw);
-}
-
-// The same for FP32 by the strip solve of warp_solve.cuh: strip j of a block's inverse is
-// zero above row 32 j, so it solves only the trailing rows.  Eight warps per strip: the first
-// strip's 120 tiles are bound by shared-memory reads, its diagonal blocks by their chain
-// (four blocks of 512 rows: 0.060 ms, 0.125 with block_solve_strip; 4 / 8 / 12 / 16
-// warps for the strsm adjoint of order 2048 with 512 right-hand sides: 0.280 / 0.270 /
-// 0.292 / 0.295 ms, 0.336 before).
+// W (m x NBI, column-major, ldw) block b := inv(op(A)_bb): blockIdx.y = b, blockIdx.x = 32-column strip
+// of the block, solved against identity columns (warp_solve.cuh, warp_invert_f64.cuh).  Strip j is
+// zero above row 32 j, so it solves only the trailing rows.
+constexpr int INV_RB = ws::RB;
+static_assert(ws::RB == wd::RB, "one block size");
+constexpr int INV_MAXBLK = 512 / INV_RB;  // blocks of up to 512 rows
+// FP32: eight warps per strip; the first strip's 120 tiles are bound by shared-memory reads, its
+// diagonal blocks by their chain (four blocks of 512 rows: 0.060 ms, against 0.125 for 64-row
+// sub-blocks with eight lanes per column; 4 / 8 / 12 / 16 warps for the strsm adjoint of order 2048
+// with 512 right-hand sides, then 0.336 ms: 0.280 / 0.270 / 0.292 / 0.295).
 constexpr int INV_WARPS = 8;
-constexpr int INV_MAXBLK = 512 / ws::RB;  // blocks of up to 512 rows
 constexpr int INV_SMEM = (INV_MAXBLK + 2 * INV_WARPS) * ws::SLOT * int(sizeof(float));
+// FP64: six warps, as many as the slots of 8 KB leave room for (eight blocks of 512 rows: 0.077 ms,
+// against 0.130 for 64-row sub-blocks).
+constexpr int INV64_WARPS = 6;
+constexpr int INV64_SMEM = (INV_MAXBLK + 2 * INV64_WARPS) * wd::SLOT * int(sizeof(double));
+
+// A strip's place in its block, in solve order (an upper block reversed along both dimensions);
+// writes the strip's zeros.
+template <typename T>
+struct InvStrip {
+    const T* a;
+    i64 sr, sl;
+    T* w;
+    i64 dir, ldw;
+    int n, cols;
+    __device__ __forceinline__ InvStrip(i64 m, int nbi, const T* A, i64 lda, bool lower, bool trans, T* W, i64 ldw_) {
+        const i64 r0 = i64(blockIdx.y) * nbi, c0 = i64(blockIdx.x) * INV_RB;
+        const int nbb = int(min(i64(nbi), m - r0));
+        n = nbb - int(c0);
+        cols = min(INV_RB, n);
+        if (n <= 0) return;
+        dir = lower ? 1 : -1;
+        ldw = dir * ldw_;
+        sr = dir * (trans ? lda : 1);
+        sl = dir * (trans ? 1 : lda);
+        a = A + r0 * (lda + 1) + (lower ? 0 : (nbb - 1) * (lda + 1)) + c0 * (sr + sl);
+        T* const w00 = W + r0 + (lower ? 0 : (nbb - 1) * (ldw_ + 1));
+        w = w00 + c0 * (dir + ldw);
+        for (int r = threadIdx.x; r < c0; r += blockDim.x) {
+            T* q = w00 + dir * r + c0 * ldw;
+            for (int c = 0; c < cols; ++c, q += ldw) *q = T(0);
+        }
+    }
+};
+
 __global__ void __launch_bounds__(32 * INV_WARPS, 1)
 block_invert_f32_kernel(i64 m, int nbi, const float* __restrict__ A, i64 lda, bool lower, bool trans, bool unit,
                         float* __restrict__ W, i64 ldw, int* err) {
@@ -431,31 +453,30 @@ block_invert_f32_kernel(i64 m, int nbi, const float* __restrict__ A, i64 lda, bo
     __shared__ uint64_t bars[INV_MAXBLK];
     pdl_next();
     pdl_wait();
-    const i64 r0 = i64(blockIdx.y) * nbi;
-    const int nbb = int(min(i64(nbi), m - r0)), c0 = int(blockIdx.x) * ws::RB;
-    if (c0 >= nbb) return;
+    const InvStrip<float> s(m, nbi, A, lda, lower, trans, W, ldw);
+    if (s.n <= 0) return;
     if (threadIdx.x < INV_MAXBLK) tc::mbar_init(&bars[threadIdx.x], 1);
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // the block in solve order: an upper one reversed along both dimensions
-    const i64 dir = lower ? 1 : -1;
-    float* const w00 = W + r0 + (lower ? 0 : (nbb - 1) * (ldw + 1));
-    ws::Problem p;
-    ws::solve_order(p, A + r0 * (lda + 1), lda, nbb, lower, trans);
-    p.a += c0 * (p.sr + p.sl);
-    p.n = nbb - c0;
-    p.b = w00 + c0 * dir * (ldw + 1);
-    p.sb = dir;
-    p.ldb = dir * ldw;
-    p.cols = min(ws::RB, p.n);
-    p.alpha = 1.0f;
-    p.unit = unit;
-    for (int r = 32 * warp; r < c0; r += 32 * INV_WARPS) {
-        float* q = w00 + dir * (r + lane) + dir * c0 * ldw;
-        for (int c = 0; c < p.cols; ++c, q += dir * ldw) *q = 0.0f;
-    }
+    const ws::Problem p{s.a, s.sr, s.sl, s.w, s.dir, s.ldw, s.n, s.cols, 1.0f, unit};
     ws::solve_strip<true>(p, warp, INV_WARPS, inv_smem, inv_smem + (INV_MAXBLK + 2 * warp) * ws::SLOT, bars, nullptr, lane,
                           err);
+}
+
+__global__ void __launch_bounds__(32 * INV64_WARPS, 1)
+block_invert_f64_kernel(i64 m, int nbi, const double* __restrict__ A, i64 lda, bool lower, bool trans, bool unit,
+                        double* __restrict__ W, i64 ldw, int* err) {
+    extern __shared__ __align__(16) double inv_smem64[];
+    __shared__ uint64_t bars[INV_MAXBLK];
+    pdl_next();
+    pdl_wait();
+    const InvStrip<double> s(m, nbi, A, lda, lower, trans, W, ldw);
+    if (s.n <= 0) return;
+    if (threadIdx.x < INV_MAXBLK) tc::mbar_init(&bars[threadIdx.x], 1);
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const wd::Strip p{s.a, s.sr, s.sl, s.w, s.dir, s.ldw, s.n, s.cols, unit};
+    wd::invert_strip(p, warp, INV64_WARPS, inv_smem64, inv_smem64 + (INV_MAXBLK + 2 * warp) * wd::SLOT, bars, lane, err);
 }
 
 template <typename T>
@@ -463,35 +484,23 @@ i64 inv_block_rows() {  // the tuning table's 256 or 512 (<= bs_max_rows<T>() fo
     return tuning().trsm_inverse_block == 256 ? 256 : 512;
 }
 
-template <typename T, bool L, bool TR, bool U>
-int launch_block_invert_t(i64 m, int nbi, const T* a, i64 lda, T* w, i64 ldw) {
-    auto kern = block_invert_kernel<T, L, TR, U>;
+template <typename T>
+int launch_block_invert(bool lower, bool trans, bool unit, i64 m, int nbi, const T* a, i64 lda, T* w, i64 ldw) {
+    constexpr bool F32 = sizeof(T) == 4;
+    constexpr int smem = F32 ? INV_SMEM : INV64_SMEM;
+    void (*kern)(i64, int, const T*, i64, bool, bool, bool, T*, i64, int*);
+    if constexpr (F32) kern = block_invert_f32_kernel;
+    else kern = block_invert_f64_kernel;
     static std::atomic<unsigned> configured{0};  // one bit per device
     int dev = 0;
     MBG_CUDA(cudaGetDevice(&dev));
     if (!configured_on(configured, dev)) {
-        MBG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)bs_smem_bytes<T>(bs_max_rows<T>())));
+        MBG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         mark_configured(configured, dev);
     }
-    const dim3 g(unsigned(cdiv(nbi, BS_COLS)), unsigned(cdiv(m, nbi)));
-    MBG_CUDA(launch_pdl(kern, g, dim3(BS_THREADS), bs_smem_bytes<T>(nbi), stream(), m, nbi, a, lda, w, ldw));
-    return check_launch("trsm_block_invert");
-}
-
-int launch_block_invert_f32(bool lower, bool trans, bool unit, i64 m, int nbi, const float* a, i64 lda, float* w,
-                            i64 ldw) {
-    static std::atomic<unsigned> configured{0};  // one bit per device
-    int dev = 0;
-    MBG_CUDA(cudaGetDevice(&dev));
-    if (!configured_on(configured, dev)) {
-        MBG_CUDA(cudaFuncSetAttribute(block_invert_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      INV_SMEM));
-        mark_configured(configured, dev);
-    }
-    const dim3 g(unsigned(cdiv(nbi, ws::RB)), unsigned(cdiv(m, nbi)));
-    MBG_CUDA(launch_pdl(block_invert_f32_kernel, g, dim3(32 * INV_WARPS), INV_SMEM, stream(), m, nbi, a, lda, lower, trans,
-                        unit, w, ldw, device_error_flag()));
+    const dim3 g(unsigned(cdiv(nbi, INV_RB)), unsigned(cdiv(m, nbi)));
+    MBG_CUDA(launch_pdl(kern, g, dim3(32 * (F32 ? INV_WARPS : INV64_WARPS)), size_t(smem), stream(), m, nbi, a, lda, lower,
+                        trans, unit, w, ldw, device_error_flag()));
     return check_launch("trsm_block_invert");
 }
 
@@ -506,19 +515,7 @@ int invert_diagonal_blocks(bool lower, bool trans, bool unit, i64 m, int nbi, co
     if (nb_last < nbi)
         MBG_CUDA(cudaMemset2DAsync(w + r_last + nb_last * m, size_t(m) * sizeof(T), 0, size_t(nb_last) * sizeof(T),
                                    size_t(nbi - nb_last), stream()));
-    if constexpr (sizeof(T) == 4) {
-        return launch_block_invert_f32(lower, trans, unit, m, nbi, a, lda, w, m);
-    } else {
-#define BIV(L, TR, U) return launch_block_invert_t<T, L, TR, U>(m, nbi, a, lda, w, m)
-        if (lower) {
-            if (trans) { if (unit) BIV(true, true, true); else BIV(true, true, false); }
-            else { if (unit) BIV(true, false, true); else BIV(true, false, false); }
-        } else {
-            if (trans) { if (unit) BIV(false, true, true); else BIV(false, true, false); }
-            else { if (unit) BIV(false, false, true); else BIV(false, false, false); }
-        }
-#undef BIV
-    }
+    return launch_block_invert<T>(lower, trans, unit, m, nbi, a, lda, w, m);
 }
 
 // The inverses' planes (bf16 split terms or Ozaki slices), made once per solve.

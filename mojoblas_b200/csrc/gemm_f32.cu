@@ -95,23 +95,22 @@ int launch_f32_ck(int S, bool ta, bool tb, i64 m, i64 n, i64 k, float alpha, con
 }
 
 // Tile and CTAs per tile of a product under two waves of 128-tiles, by the estimated time in
-// microseconds.  A 16-deep slab takes the longer of a CTA's own latency and its share of the SM:
-// 0.51 and 0.46 for 64-tiles, 1.54 for 128-tiles, and 0.74, 0.64 and 1.76 where neither operand
-// takes 16-byte copies; sharing a tile adds 1 + 0.2 S, and has to be worth a tenth.  (Measured
-// around each call, launch included: 512^3 NT 26.9 us on 64-tiles, 17.7 with four CTAs each, 19.6 on
-// 128-tiles with six; 64 x 64 x 1000 TT 54.9 and, with eight, 14.7; 1000^3 NN 91 on 64-tiles, 68 on
-// 128-tiles with two.)
+// microseconds.  A slab takes the longer of a CTA's own latency and its share of the SM: 0.51 and
+// 0.46 for 64-tiles (16 deep), 2.75 for 128-tiles (32 deep), and 0.74, 0.64 and 3.15 where neither
+// operand takes 16-byte copies; sharing a tile adds 1 + 0.2 S, and has to be worth a tenth.
+// (Measured around each call, launch included: 512^3 NT 26.9 us on 64-tiles, 17.7 with four CTAs
+// each; 64 x 64 x 1000 TT 54.9 and, with eight, 14.7; 1000^3 NN 91 on 64-tiles, 68 on 128-tiles
+// with two.)
 struct F32Shape {
     int ft, S;
 };
 inline F32Shape f32_shape(i64 m, i64 n, i64 k, int vec_operands, bool may_share) {
     F32Shape best{64, 1};
     double t_best = 0;
-    const i64 slabs = cdiv(k, FK);
     const double scalar = (2 - vec_operands) / 2.0;
     for (int ft = 64; ft <= 128; ft *= 2) {
-        const i64 tiles = cdiv(m, ft) * cdiv(n, ft);
-        const double lat = ft == 128 ? 1.54 + 0.22 * scalar : 0.51 + 0.23 * scalar;
+        const i64 tiles = cdiv(m, ft) * cdiv(n, ft), slabs = cdiv(k, ft == 128 ? FTile<128>::K : FTile<64>::K);
+        const double lat = ft == 128 ? 2.75 + 0.4 * scalar : 0.51 + 0.23 * scalar;
         const double rate = ft == 128 ? lat : 0.46 + 0.18 * scalar;
         for (int S = 1; S <= (may_share ? clu::MAX_CTAS : 1) && S <= slabs; ++S) {
             const double share = rate * double(cdiv(tiles * S, clu::usable_sms(S)));

@@ -5,8 +5,8 @@
 // block per thread, rows tx*4+{0..3} and 64+tx*4+{0..3}, columns likewise from
 // ty; FT = 64: 4 x 4), one FMA per product (two products per fma.rn.f32x2
 // instruction), each element's sum running over k in ascending order as in the
-// reference's column loops.  K advances in slabs of 16
-// through a 3-stage cp.async pipeline straight into shared memory: an operand
+// reference's column loops.  K advances in slabs (32 deep in two stages for 128-tiles, 16 in
+// three for 64-tiles) through a cp.async pipeline straight into shared memory: an operand
 // contiguous along m (n), 16-byte aligned with ld % 4 == 0, is copied 16 bytes
 // at a time, any other operand element by element into the same k-major tiles
 // (rows padded to FT + 4 floats).  beta == 0 writes C without reading it,
@@ -20,10 +20,15 @@
 namespace mbg {
 namespace f32t {
 
-constexpr int FK = 16, FSTAGES = 3, FNT = 256;
+constexpr int FNT = 256;
 template <int FT> struct FTile {
     static constexpr int LD = FT + 4;     // tile row (floats)
     static constexpr int TM = FT / 16;    // rows (and columns) per thread: 8 or 4
+    // slab depth and stages: between slabs the FP32 pipe waits for a barrier and first loads, so
+    // 128-tiles take deep ones (sgemm NT 4096^3: 16 x 3 stages 2.62 ms, 16 x 4 2.52, 24 x 3 2.54, 8 x 4
+    // 2.48, 32 x 3 2.37, 32 x 2 2.36); 64-tiles keep short reductions divisible among CTAs
+    static constexpr int K = FT == 128 ? 32 : 16;
+    static constexpr int STAGES = FT == 128 ? 2 : 3;
 };
 
 __device__ __forceinline__ void cpa4(void* dst, const void* src, bool valid) {
@@ -61,13 +66,13 @@ __device__ __forceinline__ void f32_tri_tile(i64 t, i64& ti, i64& tj) {
     tj = t - r * (r + 1) / 2;
 }
 
-// Copies one FK-deep slab of an operand into a [k][FLD] tile.  MAJ: the operand
+// Copies one slab of an operand into a [k][FLD] tile.  MAJ: the operand
 // is contiguous along the tile's row index (m or n) in memory; else along k.
 // VEC: 16-byte copies along the contiguous index.
 template <int FT, bool MAJ, bool VEC>
 __device__ __forceinline__ void f32_stage(float* tile, const float* __restrict__ P, i64 ld, i64 r0, i64 rows,
                                           i64 k0, i64 k, int tid) {
-    constexpr int FLD = FTile<FT>::LD;
+    constexpr int FLD = FTile<FT>::LD, FK = FTile<FT>::K;
     if (MAJ && VEC) {  // 4 consecutive rows of one k per copy
 #pragma unroll
         for (int e0 = tid; e0 < FT * FK / 4; e0 += FNT) {
@@ -99,7 +104,7 @@ template <int FT, bool TA, bool TB, int TRI, bool VA, bool VB, bool CK = false>
 __device__ __forceinline__ void f32_tile(i64 m, i64 n, i64 k, float alpha, const float* __restrict__ A, i64 lda,
                                          const float* __restrict__ B, i64 ldb, float beta, float* __restrict__ C,
                                          i64 ldc, i64 tm, i64 tn, float* fsm, int band = KB_NONE) {
-    constexpr int FLD = FTile<FT>::LD, TM = FTile<FT>::TM;
+    constexpr int FLD = FTile<FT>::LD, TM = FTile<FT>::TM, FK = FTile<FT>::K, FSTAGES = FTile<FT>::STAGES;
     float* As = fsm;                               // [stage][k][FLD]
     float* Bs = fsm + size_t(FSTAGES) * FK * FLD;  // [stage][k][FLD]
     const i64 m0 = tm * FT, n0 = tn * FT;
@@ -242,7 +247,7 @@ __device__ __forceinline__ void f32_tile(i64 m, i64 n, i64 k, float alpha, const
 }
 
 template <int FT>
-constexpr size_t f32_smem() { return sizeof(float) * size_t(FSTAGES) * FK * FTile<FT>::LD * 2; }
+constexpr size_t f32_smem() { return sizeof(float) * size_t(FTile<FT>::STAGES) * FTile<FT>::K * FTile<FT>::LD * 2; }
 
 template <int FT>
 constexpr size_t f32_ck_smem() { return f32_smem<FT>() > sizeof(float) * FT * FT ? f32_smem<FT>() : sizeof(float) * FT * FT; }

@@ -109,7 +109,7 @@ inline F32Shape f32_shape(i64 m, i64 n, i64 k, int vec_operands, bool may_share)
     double t_best = 0;
     const double scalar = (2 - vec_operands) / 2.0;
     for (int ft = 64; ft <= 128; ft *= 2) {
-        const i64 tiles = cdiv(m, ft) * cdiv(n, ft), slabs = cdiv(k, ft == 128 ? FTile<128>::K : FTile<64>::K);
+        const i64 tiles = cdiv(m, ft) * cdiv(n, ft), slabs = cdiv(k, ft == 128 ? Deep<128>::K : Deep<64>::K);
         const double lat = ft == 128 ? 2.75 + 0.4 * scalar : 0.51 + 0.23 * scalar;
         const double rate = ft == 128 ? lat : 0.46 + 0.18 * scalar;
         for (int S = 1; S <= (may_share ? clu::MAX_CTAS : 1) && S <= slabs; ++S) {

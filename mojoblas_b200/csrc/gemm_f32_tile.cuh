@@ -24,11 +24,16 @@ constexpr int FNT = 256;
 template <int FT> struct FTile {
     static constexpr int LD = FT + 4;     // tile row (floats)
     static constexpr int TM = FT / 16;    // rows (and columns) per thread: 8 or 4
-    // slab depth and stages: between slabs the FP32 pipe waits for a barrier and first loads, so
-    // 128-tiles take deep ones (sgemm NT 4096^3: 16 x 3 stages 2.62 ms, 16 x 4 2.52, 24 x 3 2.54, 8 x 4
-    // 2.48, 32 x 3 2.37, 32 x 2 2.36); 64-tiles keep short reductions divisible among CTAs
-    static constexpr int K = FT == 128 ? 32 : 16;
-    static constexpr int STAGES = FT == 128 ? 2 : 3;
+};
+// Slab depth and stages.  Between slabs the FP32 pipe waits for a barrier and first loads, so 128-tiles
+// take deep ones (sgemm NT 4096^3: 16 x 3 stages 2.62 ms, 16 x 4 2.52, 24 x 3 2.54, 8 x 4 2.48, 32 x 3
+// 2.37, 32 x 2 2.36); 64-tiles keep short reductions divisible among CTAs, and grouped plans
+// (Shallow) theirs from being padded (4096 problems of 16..512 on 32 x 2: 1.69 ms against 1.62).
+template <int FT> struct Deep {
+    static constexpr int K = FT == 128 ? 32 : 16, STAGES = FT == 128 ? 2 : 3;
+};
+struct Shallow {
+    static constexpr int K = 16, STAGES = 3;
 };
 
 __device__ __forceinline__ void cpa4(void* dst, const void* src, bool valid) {
@@ -69,10 +74,10 @@ __device__ __forceinline__ void f32_tri_tile(i64 t, i64& ti, i64& tj) {
 // Copies one slab of an operand into a [k][FLD] tile.  MAJ: the operand
 // is contiguous along the tile's row index (m or n) in memory; else along k.
 // VEC: 16-byte copies along the contiguous index.
-template <int FT, bool MAJ, bool VEC>
+template <int FT, int FK, bool MAJ, bool VEC>
 __device__ __forceinline__ void f32_stage(float* tile, const float* __restrict__ P, i64 ld, i64 r0, i64 rows,
                                           i64 k0, i64 k, int tid) {
-    constexpr int FLD = FTile<FT>::LD, FK = FTile<FT>::K;
+    constexpr int FLD = FTile<FT>::LD;
     if (MAJ && VEC) {  // 4 consecutive rows of one k per copy
 #pragma unroll
         for (int e0 = tid; e0 < FT * FK / 4; e0 += FNT) {
@@ -100,11 +105,11 @@ __device__ __forceinline__ void f32_stage(float* tile, const float* __restrict__
 // CK: the CTAs of a cluster share the tile, each taking an equal part of the slabs; each then
 // leaves its sums in its shared memory (f32_ck_smem<FT>() bytes in all) and adds up its share
 // of the columns over the cluster, in the CTAs' order, so results do not depend on scheduling.
-template <int FT, bool TA, bool TB, int TRI, bool VA, bool VB, bool CK = false>
+template <int FT, bool TA, bool TB, int TRI, bool VA, bool VB, bool CK = false, class Slab = Deep<FT>>
 __device__ __forceinline__ void f32_tile(i64 m, i64 n, i64 k, float alpha, const float* __restrict__ A, i64 lda,
                                          const float* __restrict__ B, i64 ldb, float beta, float* __restrict__ C,
                                          i64 ldc, i64 tm, i64 tn, float* fsm, int band = KB_NONE) {
-    constexpr int FLD = FTile<FT>::LD, TM = FTile<FT>::TM, FK = FTile<FT>::K, FSTAGES = FTile<FT>::STAGES;
+    constexpr int FLD = FTile<FT>::LD, TM = FTile<FT>::TM, FK = Slab::K, FSTAGES = Slab::STAGES;
     float* As = fsm;                               // [stage][k][FLD]
     float* Bs = fsm + size_t(FSTAGES) * FK * FLD;  // [stage][k][FLD]
     const i64 m0 = tm * FT, n0 = tn * FT;
@@ -112,8 +117,8 @@ __device__ __forceinline__ void f32_tile(i64 m, i64 n, i64 k, float alpha, const
 
     // op(A) is m-contiguous when A is not transposed; op(B) is n-contiguous when B is
     auto issue = [&](i64 kt, int st) {
-        f32_stage<FT, !TA, VA>(As + size_t(st) * FK * FLD, A, lda, m0, m, kt * FK, k, tid);
-        f32_stage<FT, TB, VB>(Bs + size_t(st) * FK * FLD, B, ldb, n0, n, kt * FK, k, tid);
+        f32_stage<FT, FK, !TA, VA>(As + size_t(st) * FK * FLD, A, lda, m0, m, kt * FK, k, tid);
+        f32_stage<FT, FK, TB, VB>(Bs + size_t(st) * FK * FLD, B, ldb, n0, n, kt * FK, k, tid);
     };
 
     // accumulators in pairs of adjacent columns: accp[i][jp] = (acc[i][2 jp], acc[i][2 jp + 1])
@@ -246,8 +251,8 @@ __device__ __forceinline__ void f32_tile(i64 m, i64 n, i64 k, float alpha, const
     }
 }
 
-template <int FT>
-constexpr size_t f32_smem() { return sizeof(float) * size_t(FTile<FT>::STAGES) * FTile<FT>::K * FTile<FT>::LD * 2; }
+template <int FT, class Slab = Deep<FT>>
+constexpr size_t f32_smem() { return sizeof(float) * size_t(Slab::STAGES) * Slab::K * FTile<FT>::LD * 2; }
 
 template <int FT>
 constexpr size_t f32_ck_smem() { return f32_smem<FT>() > sizeof(float) * FT * FT ? f32_smem<FT>() : sizeof(float) * FT * FT; }

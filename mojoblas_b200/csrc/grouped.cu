@@ -48,7 +48,7 @@ template <int TILE, bool TA, bool TB>
 __device__ __forceinline__ void grouped_tile(const GemmDesc& d, i64 tm, i64 tn, float* gsm) {
     const bool va = f32t::f32_vec(!TA, d.a, d.lda), vb = f32t::f32_vec(TB, d.b, d.ldb);
 #define GT(VA, VB) \
-    f32t::f32_tile<TILE, TA, TB, 0, VA, VB>(d.m, d.n, d.k, d.alpha, d.a, d.lda, d.b, d.ldb, d.beta, d.c, d.ldc, tm, tn, gsm)
+    f32t::f32_tile<TILE, TA, TB, 0, VA, VB, false, f32t::Shallow>(d.m, d.n, d.k, d.alpha, d.a, d.lda, d.b, d.ldb, d.beta, d.c, d.ldc, tm, tn, gsm)
     if (va && vb) GT(true, true);
     else if (va) GT(true, false);
     else if (vb) GT(false, true);
@@ -60,7 +60,7 @@ template <int TILE>
 __global__ void __launch_bounds__(GT_NT, TILE == 128 ? 1 : 3)
 grouped_sgemm_kernel(const GemmDesc* __restrict__ probs, int count, i64 total_tiles,
                      unsigned long long* __restrict__ counter) {
-    extern __shared__ __align__(16) float gsm[];  // f32t::f32_smem<TILE>() bytes
+    extern __shared__ __align__(16) float gsm[];  // f32t::f32_smem<TILE, Shallow>() bytes
     __shared__ long long s_tile;
     for (;;) {
         if (threadIdx.x == 0) s_tile = (long long)atomicAdd(counter, 1ull);
@@ -234,13 +234,13 @@ int enqueue_plan(mbg_plan* p, cudaStream_t s) {
         // the 128-tile problems (the larger size classes) first, the 64-tile ones behind them
         if (p->count128 > 0) {
             MBG_CUDA(cudaMemsetAsync(p->counter128, 0, sizeof(unsigned long long), s));
-            grouped_sgemm_kernel<128><<<p->grid128, GT_NT, f32t::f32_smem<128>(), s>>>(
+            grouped_sgemm_kernel<128><<<p->grid128, GT_NT, f32t::f32_smem<128, f32t::Shallow>(), s>>>(
                 static_cast<const GemmDesc*>(p->table128), p->count128, p->total128, p->counter128);
             MBG_TRY(check_launch("grouped_sgemm"));
         }
         if (p->count > 0) {
             MBG_CUDA(cudaMemsetAsync(p->counter, 0, sizeof(unsigned long long), s));
-            grouped_sgemm_kernel<64><<<p->grid, GT_NT, f32t::f32_smem<64>(), s>>>(
+            grouped_sgemm_kernel<64><<<p->grid, GT_NT, f32t::f32_smem<64, f32t::Shallow>(), s>>>(
                 static_cast<const GemmDesc*>(p->table), p->count, p->total, p->counter);
             MBG_TRY(check_launch("grouped_sgemm"));
         }
@@ -363,12 +363,12 @@ int mbg_sgemm_grouped_plan(int mode, int count, const mbg_sgemm_problem* probs, 
     int per_sm64 = 1, per_sm128 = 1;
     // dynamic shared memory above 48 KB needs the opt-in before the occupancy query and the launch
     cudaFuncSetAttribute(grouped_sgemm_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         int(f32t::f32_smem<128>()));
+                         int(f32t::f32_smem<128, f32t::Shallow>()));
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm128, grouped_sgemm_kernel<128>, GT_NT,
-                                                  f32t::f32_smem<128>());
+                                                  f32t::f32_smem<128, f32t::Shallow>());
     cudaFuncSetAttribute(grouped_sgemm_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         int(f32t::f32_smem<64>()));
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm64, grouped_sgemm_kernel<64>, GT_NT, f32t::f32_smem<64>());
+                         int(f32t::f32_smem<64, f32t::Shallow>()));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm64, grouped_sgemm_kernel<64>, GT_NT, f32t::f32_smem<64, f32t::Shallow>());
     cudaGetLastError();
     p->grid = int(imax(1, imin(tiles[0], i64(num_sms()) * imax(per_sm64, 1))));
     p->grid128 = int(imax(1, imin(tiles[1], i64(num_sms()) * imax(per_sm128, 1))));

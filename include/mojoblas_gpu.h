@@ -268,7 +268,7 @@ int mbg_dtrsm_adjoint(int mode, int slices, char side, char uplo, char trans_a, 
  *          shared memory (no pre-pass, any leading dimension), tiles of 128 x 64
  *          or 128 x 128 per problem (tuning table), longest reduction first.
  *   strsm: side 'L' only, m <= 256 (the triangle order), any uplo/trans/diag;
- *          32-column strips solved by the fused diagonal-block routine;
+ *          32-column strips, each solved by one, two or four warps;
  *          mode MBG_MODE_PLAIN. */
 typedef struct {
     char trans_a, trans_b;

@@ -391,7 +391,7 @@ int launch_copy(i64 m, i64 n, T alpha, const T* x, i64 ldx, T* y, i64 ldy) {
 
 // ---- inverted diagonal blocks (split / Ozaki modes) ---------------------------------
 // The split / Ozaki solve: every diagonal block of NBI rows is inverted once in the
-// input precision (fused block solves of the identity, all blocks in one launch), the
+// input precision (strips of the identity solved in shared memory, all blocks in one launch), the
 // inverses' planes are made once, and the solve recurses as solve_left does, except that
 // each leaf is one product X_b = inv(op(A)_bb) B_b on the tensor cores instead of a
 // substitution.  So every flop of the solve runs in split / Ozaki products: the leaves'

@@ -39,6 +39,7 @@
 // producer warps, and branches around each column of the epilogue's stores.
 #include "mbg_internal.cuh"
 #include "gemm_f32_tile.cuh"
+#include "schedule.cuh"
 #include "tc_ptx.cuh"
 
 #include <cuda_bf16.h>
@@ -85,25 +86,25 @@ struct __align__(16) TcTile {
     const float* b;  // the tile's first column
     float* c;        // the tile's corner
     i64 lda, ldb, ldc;
-    int k, nkb;      // nkb: k slabs (0 when alpha == 0 or k == 0: C := beta C only)
+    int nkb, last;   // k slabs (0 when alpha == 0 or k == 0: C := beta C only), elements of the last
     int rows, cols;  // of the tile inside the problem
     int bn;          // tile columns: 64 or 128
     int kcontig;     // bit 0: op(A)'s k is the contiguous dimension, bit 1: op(B)'s
     float alpha, beta;
 };
 
-// A warp's 32 rows (rw0 ..) of a k slab as 16 k-adjacent pairs per lane: pair i is k (2 i, 2 i + 1) of
-// row rw0 + lane, or, KC (k contiguous), k (2 q, 2 q + 1) of row rw0 + 2 i + h with (h, q) =
-// (lane / 16, lane % 16), so that a load covers two rows of 128 bytes.  Zeros past the
-// operand's rows and past K.
+// A warp's 32 rows (rw0 ..) of a k slab, `left` deep from p on, as 16 k-adjacent pairs per lane: pair i
+// is k (2 i, 2 i + 1) of row rw0 + lane, or, KC (k contiguous), k (2 q, 2 q + 1) of row
+// rw0 + 2 i + h with (h, q) = (lane / 16, lane % 16), so that a load covers two rows of 128 bytes.
+// Zeros past the operand's rows and past the slab's end.
 template <bool KC>
-__device__ __forceinline__ void load_pairs(float (&v)[32], const float* __restrict__ p, i64 ld, int rw0, int rows, int k0,
-                                           int K, int lane) {
+__device__ __forceinline__ void load_pairs(float (&v)[32], const float* __restrict__ p, i64 ld, int rw0, int rows,
+                                           int left, int lane) {
     if (KC) {
-        const int h = lane >> 4, k = k0 + 2 * (lane & 15);
+        const int h = lane >> 4, k = 2 * (lane & 15);
         const float* q = p + i64(rw0 + h) * ld + k;
-        const bool on0 = k < K, on1 = k + 1 < K;
-        if (rw0 + 32 <= rows && k0 + 32 <= K) {
+        const bool on0 = k < left, on1 = k + 1 < left;
+        if (rw0 + 32 <= rows && left == GBK) {
 #pragma unroll
             for (int i = 0; i < 16; ++i, q += 2 * ld) {
                 v[2 * i] = __ldg(q);
@@ -118,14 +119,14 @@ __device__ __forceinline__ void load_pairs(float (&v)[32], const float* __restri
             }
         }
     } else {
-        const float* q = p + rw0 + lane + i64(k0) * ld;
+        const float* q = p + rw0 + lane;
         const bool r = rw0 + lane < rows;
-        if (k0 + 32 <= K) {
+        if (left == GBK) {
 #pragma unroll
             for (int l = 0; l < 32; ++l, q += ld) v[l] = r ? __ldg(q) : 0.0f;
         } else {
 #pragma unroll
-            for (int l = 0; l < 32; ++l, q += ld) v[l] = r && k0 + l < K ? __ldg(q) : 0.0f;
+            for (int l = 0; l < 32; ++l, q += ld) v[l] = r && l < left ? __ldg(q) : 0.0f;
         }
     }
 }
@@ -230,15 +231,15 @@ grouped_tc_kernel(const TcTile* __restrict__ tiles, int ntiles, int* err) {
         const int plane_bytes = isA ? C::A_PLANE : C::B_PLANE;
         int it = 0;  // slabs of this CTA before the current tile
         bool ok = true;
-        struct View { const float* p; i64 ld; int K, nkb, rows, used, kc; };
+        struct View { const float* p; i64 ld; int nkb, last, rows, used, kc; };
         auto view = [&](int t) {
             View o{};
             if (t < ntiles) {
                 const TcTile* d = tiles + t;
                 o.p = isA ? d->a : d->b;
                 o.ld = isA ? d->lda : d->ldb;
-                o.K = d->k;
                 o.nkb = d->nkb;
+                o.last = d->last;
                 o.rows = isA ? d->rows : d->cols;
                 o.used = isA ? BM : d->bn;
                 o.kc = (d->kcontig >> (isA ? 0 : 1)) & 1;
@@ -249,17 +250,20 @@ grouped_tc_kernel(const TcTile* __restrict__ tiles, int ntiles, int* err) {
         for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
             const View o = next;
             next = view(t + gridDim.x);  // a tile ahead
-            for (int kb = (it ^ group) & 1; kb < o.nkb; kb += GGROUPS) {
+            const i64 slab = o.kc ? i64(GBK) : GBK * o.ld;  // from one slab's start to the next's
+            const float* p = o.p + ((it ^ group) & 1) * slab;
+            for (int kb = (it ^ group) & 1; kb < o.nkb; kb += GGROUPS, p += GGROUPS * slab) {
                 const int s = (it + kb) % C::STAGES, use = (it + kb) / C::STAGES;
                 uint8_t* const plane0 = planes + s * C::STAGE_BYTES;
                 if (rw0 < o.rows) {
                     float v[32];
+                    const int left = k_left(o.nkb, o.last, kb, GBK);
                     if (o.kc) {
-                        load_pairs<true>(v, o.p, o.ld, rw0, o.rows, kb * GBK, o.K, lane);
+                        load_pairs<true>(v, p, o.ld, rw0, o.rows, left, lane);
                         if (!mbar_wait(&empty[s], (use & 1) ^ 1, err, 31)) { ok = false; break; }
                         split_store<TERMS, true>(v, plane0, plane_bytes, rw0, lane);
                     } else {
-                        load_pairs<false>(v, o.p, o.ld, rw0, o.rows, kb * GBK, o.K, lane);
+                        load_pairs<false>(v, p, o.ld, rw0, o.rows, left, lane);
                         if (!mbar_wait(&empty[s], (use & 1) ^ 1, err, 31)) { ok = false; break; }
                         split_store<TERMS, false>(v, plane0, plane_bytes, rw0, lane);
                     }
@@ -413,8 +417,10 @@ int grouped_tc_build(int terms, int count, const mbg_sgemm_problem* probs, Group
         const bool ta = is_t(q.trans_a), tb = is_t(q.trans_b);
         const int bn = grouped_tc_tile_cols(q.m, q.n, q.k, ta, tb);
         TcTile d{};
-        d.lda = q.lda; d.ldb = q.ldb; d.ldc = q.ldc; d.k = int(q.k);
-        d.nkb = (q.alpha == 0.0f || q.k == 0) ? 0 : int(cdiv(q.k, GBK));
+        d.lda = q.lda; d.ldb = q.ldb; d.ldc = q.ldc;
+        const KSlabs slabs = k_slabs(q.alpha == 0.0f ? 0 : q.k, GBK);
+        d.nkb = int(slabs.n);
+        d.last = slabs.last;
         d.bn = bn;
         d.kcontig = (ta ? 1 : 0) | (tb ? 0 : 2);
         d.alpha = q.alpha; d.beta = q.beta;

@@ -413,12 +413,12 @@ int grouped_tc_build(int terms, int count, const mbg_sgemm_problem* probs, Group
         const mbg_sgemm_problem& q = probs[i];
         if (q.m == 0 || q.n == 0) continue;
         ++out.count;
-        if (q.k > 0x7fffffff) return MBG_ERR_UNSUPPORTED;
         const bool ta = is_t(q.trans_a), tb = is_t(q.trans_b);
         const int bn = grouped_tc_tile_cols(q.m, q.n, q.k, ta, tb);
         TcTile d{};
         d.lda = q.lda; d.ldb = q.ldb; d.ldc = q.ldc;
         const KSlabs slabs = k_slabs(q.alpha == 0.0f ? 0 : q.k, GBK);
+        if (slabs.n > 0x7fffffff) return MBG_ERR_UNSUPPORTED;  // k > 2^36: one row of op(A) takes 256 GB
         d.nkb = int(slabs.n);
         d.last = slabs.last;
         d.bn = bn;

@@ -19,8 +19,10 @@ __device__ __forceinline__ uint32_t size() {
     asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
     return r;
 }
-// Every thread of every CTA of the cluster, with its warp converged.
+// Every thread of every CTA of the cluster.  The aligned forms want a converged warp, which a loop
+// with different trips per lane, or a lane's early `continue`, does not promise.
 __device__ __forceinline__ void sync_all() {
+    __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // The address in CTA `r`'s shared memory of what sits at `addr` in this one's.

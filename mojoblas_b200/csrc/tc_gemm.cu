@@ -395,7 +395,6 @@ __device__ __forceinline__ void tc_gemm_tile(const CUtensorMap& tmA, const CUten
     }
     if constexpr (CK) {
         static_assert(BM * C::BN * 4 <= C::STAGES * C::STAGE_BYTES, "the sums reuse the stage buffers");
-        __syncwarp();
         clu::sync_all();
         if (warp >= 2) {
             const int S = int(clu::size()), r = int(clu::rank());
@@ -435,7 +434,6 @@ __device__ __forceinline__ void tc_gemm_tile(const CUtensorMap& tmA, const CUten
                                 lo, hi);
             }
         }
-        __syncwarp();
         clu::sync_all();  // no CTA leaves while another reads its sums
     }
 }
@@ -1190,7 +1188,6 @@ ozaki_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         }
     }
     tc_fence_before();
-    __syncwarp();
     clu::sync_all();  // the peer's epilogue and loads are done; no more remote barrier traffic
     if (warp == 0) {
         __syncwarp();

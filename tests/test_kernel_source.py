@@ -1,0 +1,22 @@
+"""Rules of the kernels' sources whose breach could hang or fault the device, and so has no test
+that runs it: read from the text."""
+import re
+from pathlib import Path
+
+CSRC = Path(__file__).resolve().parents[1] / "mojoblas_b200" / "csrc"
+SOURCES = {p.name: re.sub(r"//[^\n]*", "", p.read_text()) for p in sorted(CSRC.glob("*.cu*"))}
+
+
+def functions(text):
+    """(head, body) of every function whose closing brace is in the first column."""
+    for m in re.finditer(r"^(?:template|__global__|__device__|inline|int|void|static)[^;{}]*\{\n(.*?)^\}", text, re.M | re.S):
+        yield text[m.start():m.start(1)], m.group(1)
+
+
+def test_cluster_barrier_has_converged_warps():
+    """barrier.cluster's aligned forms need a converged warp: the one place that issues them sees to it."""
+    users = [name for name, text in SOURCES.items() if "barrier.cluster" in text]
+    assert users == ["cluster.cuh"]
+    bodies = [b for _, b in functions(SOURCES["cluster.cuh"]) if "barrier.cluster" in b]
+    assert len(bodies) == 1
+    assert "__syncwarp();" in bodies[0].split("barrier.cluster")[0]

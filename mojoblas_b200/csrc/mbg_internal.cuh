@@ -70,7 +70,10 @@ int check_launch(const char* name);
 // global memory: that returns once the kernel before has completed, and so, by induction, all
 // earlier work on the stream.  What comes before it (barriers, TMEM, descriptors) and the launch
 // itself then overlap the tail of the kernel before.  pdl_next() lets the next kernel start once
-// every block has called it.  Without the launch attribute both do nothing.
+// every block has called it, if that kernel has the attribute; whether this one has it makes
+// no difference to that.  A kernel that uses TMEM calls it after its allocation: the next
+// kernel's blocks could otherwise take an SM's TMEM first and, waiting for this kernel, keep it
+// from it for good.  Without the attribute pdl_wait() does nothing.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <class... P, class... A>

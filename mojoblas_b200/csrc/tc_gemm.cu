@@ -242,7 +242,6 @@ __device__ __forceinline__ void tc_gemm_tile(const CUtensorMap& tmA, const CUten
     if (P.band == KB_A_LOWER) tm = P.tiles_m - 1 - tm;
     if (P.band == KB_B_UPPER) tn = P.tiles_n - 1 - tn;
     const i64 m0 = i64(tm) * BM, n0 = i64(tn) * C::BN;
-    pdl_next();
     // tiles strictly above (below) the diagonal
     if ((P.tri == 1 && m0 + BM <= n0) || (P.tri == 2 && m0 > n0 + C::BN - 1)) {
         pdl_wait();
@@ -285,6 +284,7 @@ __device__ __forceinline__ void tc_gemm_tile(const CUtensorMap& tmA, const CUten
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_next();
     pdl_wait();
 
     if (warp == 0) {
@@ -765,7 +765,6 @@ ozaki_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     if (P.band == KB_A_LOWER) tm = P.tiles_m - 1 - tm;
     if (P.band == KB_B_UPPER) tn = P.tiles_n - 1 - tn;
     const i64 m0 = i64(tm) * BM, n0 = i64(tn) * C::BN;
-    pdl_next();
     // tiles strictly above (below) the diagonal
     if ((P.tri == 1 && m0 + BM <= n0) || (P.tri == 2 && m0 > n0 + C::BN - 1)) {
         pdl_wait();
@@ -799,6 +798,7 @@ ozaki_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_next();
     const int total = C::NPASS * nkb;
 
     if (warp == 0) {
@@ -1073,7 +1073,6 @@ ozaki_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     uint64_t* tempty = tfull + 1;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 1);
 
-    pdl_next();
     const uint32_t rank = clu::rank();  // 0: leader (issues the MMAs), 1: peer
     const int ntiles = ((P.tiles_m + 1) >> 1) * P.tiles_n;
     const int first = blockIdx.x >> 1, stride = gridDim.x >> 1;
@@ -1097,6 +1096,7 @@ ozaki_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     const uint32_t leader_tempty = peer_addr(tempty, 0);
+    pdl_next();
     pdl_wait();
 
     if (warp == 0) {
@@ -1343,7 +1343,6 @@ split_sk_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant_
     uint64_t* tempty = tfull + 2;         // [2]: epilogue finished reading a buffer
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
     int* const err = P0.err;
-    pdl_next();
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -1365,6 +1364,7 @@ split_sk_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_next();
     pdl_wait();
 
     if (warp == 0) {

@@ -20,3 +20,17 @@ def test_cluster_barrier_has_converged_warps():
     bodies = [b for _, b in functions(SOURCES["cluster.cuh"]) if "barrier.cluster" in b]
     assert len(bodies) == 1
     assert "__syncwarp();" in bodies[0].split("barrier.cluster")[0]
+
+
+def test_next_kernel_is_let_in_after_the_tmem_allocation():
+    """A dependent kernel's blocks may start once every block has called pdl_next().  Before this
+    kernel has its TMEM they could take it, and then wait for this kernel, which waits for them."""
+    seen = 0
+    for name, text in SOURCES.items():
+        for head, body in functions(text):
+            if "tmem_alloc" in body and "pdl_next" in body:
+                alloc = body.rindex("tmem_alloc")
+                ready = re.search(r"__syncthreads\(\)|clu::sync_all\(\)", body[alloc:])
+                assert ready and body.index("pdl_next") > alloc + ready.start(), (name, head)
+                seen += 1
+    assert seen == 4

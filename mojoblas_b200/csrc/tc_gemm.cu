@@ -799,6 +799,7 @@ ozaki_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     pdl_next();
+    pdl_wait();
     const int total = C::NPASS * nkb;
 
     if (warp == 0) {

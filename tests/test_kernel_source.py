@@ -34,3 +34,16 @@ def test_next_kernel_is_let_in_after_the_tmem_allocation():
                 assert ready and body.index("pdl_next") > alloc + ready.start(), (name, head)
                 seen += 1
     assert seen == 4
+
+
+def test_kernels_of_a_chain_wait_on_every_path():
+    """A kernel that lets the next one in takes part in a chain of dependent launches, whose order holds
+    because each waits for the one before: pdl_wait() follows pdl_next(), and a block that
+    leaves before that has waited too."""
+    for name, text in SOURCES.items():
+        for head, body in functions(text):
+            if "pdl_next();" not in body or "pdl_wait() {" in head:
+                continue
+            assert re.search(r"pdl_next\(\);\s*pdl_wait\(\);", body), (name, head)
+            before = body[:body.index("pdl_next();")]
+            assert all(re.search(r"pdl_wait\(\);\s*$", part) for part in before.split("return;")[:-1]), (name, head)

@@ -190,7 +190,7 @@ static int gemm_host_pipelined(int mode, int slices, char ta, char tb, i64 m, i6
     if (hb) { MBG_TRY(wb.reserve(e * size_t(br) * size_t(bc))); db = wb.as<T>(); dldb = br; }
     if (hc) { MBG_TRY(wc.reserve(e * size_t(m) * size_t(n))); dc = wc.as<T>(); dldc = m; }
 
-    const ScheduleColumns whole(n);
+    ScheduleColumns whole(n);
     const std::vector<i64> widths = pipeline_widths(n);
     struct Guard {  // on every return: the copy streams' work is ordered before the library stream's
         std::vector<cudaEvent_t> v;   // next use of the workspace blocks, then the events are destroyed
@@ -279,6 +279,7 @@ static int gemm_host_pipelined(int mode, int slices, char ta, char tb, i64 m, i6
     i64 j0 = 0;
     for (size_t blk = 0; blk < widths.size() && !st; ++blk) {
         const i64 w = widths[blk];
+        whole.first_column(j0);
         cudaEvent_t ev_in = ev[2 + 2 * blk], ev_done = ev[3 + 2 * blk];
         // op(B)[:, j0 : j0 + w] is columns j0.. of B ('N') or rows j0.. of B ('T')
         if (hb) {

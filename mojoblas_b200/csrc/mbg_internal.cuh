@@ -105,16 +105,18 @@ struct StreamScope {
     StreamScope& operator=(const StreamScope&) = delete;
 };
 
-// The pipelined host path computes a product in column blocks.  Whether, and into how many parts,
-// a reduction is divided depends on the size of the product, and has to be the same for every
-// block as for one call on device pointers, or the sums would be rounded differently: for its
-// lifetime, schedules of the calling thread's products go by `n` columns.
+// The pipelined host path computes a product in column blocks.  Whether, and where, a reduction is
+// divided depends on the size of the product, and has to be the same for every block as for one
+// call on device pointers, or the sums would be rounded differently: for its lifetime, schedules
+// of the calling thread's products go by `n` columns, of which theirs start at first_column().
 struct ScheduleColumns {
     explicit ScheduleColumns(i64 n);
     ~ScheduleColumns();
+    void first_column(i64 j);
     ScheduleColumns(const ScheduleColumns&) = delete;
 };
-i64 schedule_columns(i64 n);  // the columns to schedule for: the scope's, or n
+i64 schedule_columns(i64 n);   // the columns to schedule for: the scope's, or n
+i64 schedule_first_column();  // the product's first column among them; 0 outside a scope
 
 // Two non-blocking streams of the current device (host->device and device->host
 // copies of the pipelined host path), created on first use and kept.

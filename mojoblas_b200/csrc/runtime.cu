@@ -20,6 +20,7 @@ thread_local cudaStream_t t_stream = nullptr;  // mbg_set_thread_stream: this th
 thread_local bool t_stream_on = false;
 std::atomic<bool> g_sync{true};
 thread_local i64 t_schedule_columns = 0;      // ScheduleColumns: 0 outside its scope
+thread_local i64 t_schedule_first = 0;
 thread_local std::string g_last_error;
 std::atomic<int> g_fail_alloc_countdown{0};
 std::atomic<int64_t> g_launches{0};
@@ -207,8 +208,10 @@ int copy_streams(cudaStream_t* in, cudaStream_t* out) {
 
 // ---- device error flag ---------------------------------------------------------
 ScheduleColumns::ScheduleColumns(i64 n) { t_schedule_columns = n; }
-ScheduleColumns::~ScheduleColumns() { t_schedule_columns = 0; }
+ScheduleColumns::~ScheduleColumns() { t_schedule_columns = t_schedule_first = 0; }
+void ScheduleColumns::first_column(i64 j) { t_schedule_first = j; }
 i64 schedule_columns(i64 n) { return t_schedule_columns ? t_schedule_columns : n; }
+i64 schedule_first_column() { return t_schedule_first; }
 
 int* device_error_flag() {
     std::lock_guard<std::mutex> lk(g_mu);

@@ -40,12 +40,14 @@
 // proceeds to teardown (TMEM is always freed).
 #include "mbg_internal.cuh"
 #include "cluster.cuh"
+#include "schedule.cuh"
 #include "tc_ptx.cuh"
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
 #include <mutex>
+#include <type_traits>
 
 namespace mbg {
 
@@ -1197,25 +1199,8 @@ ozaki_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
 }
 
-// Work of one persistent split launch (split_sk_kernel): one or two products (the second:
-// the gemm adjoint's other gradient).  Tiles are numbered product 0's first, then product 1's.
-//   whole tiles:  the first dp_tiles tiles, worker (CTA) c taking tiles c, c + G, ...
-//                 (G workers); the triangle mask may skip tiles; C is stored
-//                 with beta.
-//   stream-K:     the slabs of the remaining tiles, [sk_begin, total) in slab positions
-//                 over all tiles, cut into G equal contiguous ranges, one per worker, so
-//                 the last wave leaves no SM idle.  A range runs on across tile boundaries
-//                 without draining the pipeline.  Whole tiles are stored; a tile two ranges
-//                 share is zeroed first (sk_zero_kernel) and both add their partial sums
-//                 (beta = 0 only).  Every range is at least one tile long, so no tile gets
-//                 more than two partial sums, and their fp32 sum does not depend on the
-//                 order they arrive in.
-struct SkWork {
-    int tiles0, tiles1;   // tiles of each product (tiles1 = 0: one product)
-    int nkb0, nkb1;       // k slabs of each product's tiles
-    int dp_tiles;         // leading tiles taken whole
-    i64 sk_begin, total;  // stream-K slab positions (sk_begin == total: none)
-};
+// Work of a persistent split launch: SkWork, or SkBlock for a column block of the pipelined host
+// path (schedule.cuh).
 struct SkSeg {
     int prod, tile, kb0, kb1;  // slabs [kb0, kb1) of tile `tile` of product `prod`
     i64 m0, n0;                // the tile's first row and column
@@ -1226,18 +1211,13 @@ struct SkCursor {
 };
 
 // Tile t of P (C::TILE_M x C::TILE_N; P.tiles_m counts 128-row tiles, P.tiles_n
-// TILE_N-column tiles): groups of TILE_GROUP tile rows walk the n-tiles together (L2 reuse).
+// TILE_N-column tiles).
 template <class C>
 __device__ __forceinline__ void sk_tile_origin(const Params& P, int t, i64& m0, i64& n0) {
     constexpr int R = C::TILE_M / BM;
-    const int tiles_m = (P.tiles_m + R - 1) / R;
-    const int per_group = C::TILE_GROUP * P.tiles_n;
-    const int g = t / per_group;
-    const int first_m = g * C::TILE_GROUP;
-    const int gsize = min(C::TILE_GROUP, tiles_m - first_m);
-    const int in_g = t - g * per_group;
-    m0 = i64(first_m + in_g % gsize) * C::TILE_M;
-    n0 = i64(in_g / gsize) * C::TILE_N;
+    const TileAt at = tile_at(TileGrid{(P.tiles_m + R - 1) / R, P.tiles_n, C::TILE_GROUP}, t);
+    m0 = i64(at.tm) * C::TILE_M;
+    n0 = i64(at.tn) * C::TILE_N;
 }
 
 // Stream-K slab position -> the tile holding it and the slab within it.
@@ -1253,13 +1233,20 @@ __device__ __forceinline__ void sk_locate(const SkWork& W, i64 pos, int& prod, i
 }
 
 __device__ __forceinline__ SkCursor sk_cursor(const SkWork& W, i64 worker, i64 workers) {
-    const i64 n = W.total - W.sk_begin;
     SkCursor c;
     c.u = int(worker);
     c.u_end = W.dp_tiles;
     c.step = int(workers);
-    c.pos = W.sk_begin + worker * n / workers;
-    c.end = W.sk_begin + (worker + 1) * n / workers;
+    c.pos = sk_range_begin(W, worker, workers);
+    c.end = sk_range_begin(W, worker + 1, workers);
+    return c;
+}
+__device__ __forceinline__ SkCursor sk_cursor(const SkBlock& B, i64 worker, i64 workers) {
+    SkCursor c;
+    c.u = int(worker);
+    c.u_end = B.block.tiles_m * B.block.tiles_n;
+    c.step = int(workers);
+    c.pos = c.end = 0;  // pos: where the current tile's second part starts, 0 ahead of its first
     return c;
 }
 
@@ -1291,6 +1278,22 @@ __device__ __forceinline__ bool sk_next(const SkWork& W, const Params& P0, const
     return true;
 }
 
+template <class C>
+__device__ __forceinline__ bool sk_next(const SkBlock& B, const Params& P, const Params&, SkCursor& cur, SkSeg& sg) {
+    if (cur.u >= cur.u_end) return false;
+    sg.prod = 0;
+    sg.tile = cur.u;
+    sk_tile_origin<C>(P, cur.u, sg.m0, sg.n0);
+    const int cut = cur.pos ? 0 : sk_block_cut(B, cur.u);
+    sg.kb0 = int(cur.pos);
+    sg.kb1 = cut ? cut : B.W.nkb0;
+    cur.pos = cut;
+    if (!cut) cur.u += cur.step;
+    return true;
+}
+__device__ __forceinline__ int sk_slabs(const SkWork& W, int prod) { return prod ? W.nkb1 : W.nkb0; }
+__device__ __forceinline__ int sk_slabs(const SkBlock& B, int) { return B.W.nkb0; }
+
 // Zeroes the tiles two stream-K ranges share, ahead of their partial sums: block b takes
 // the boundary between ranges b and b + 1 (a boundary inside a tile; ranges are at least
 // a tile long, so each such tile holds one boundary), SK_ZERO_CTAS blocks per tile (one block
@@ -1300,8 +1303,7 @@ template <class C>
 __global__ void __launch_bounds__(256) sk_zero_kernel(Params P0, Params P1, SkWork W, int workers) {
     pdl_next();
     pdl_wait();
-    const i64 n = W.total - W.sk_begin;
-    const i64 pos = W.sk_begin + (i64(blockIdx.x) + 1) * n / workers;
+    const i64 pos = sk_range_begin(W, i64(blockIdx.x) + 1, workers);
     int prod, tile, kb, nkb;
     i64 base;
     sk_locate(W, pos, prod, tile, kb, base, nkb);
@@ -1331,11 +1333,12 @@ __device__ __forceinline__ void split_add_row(const Params& P, const i64 row, co
 // and buffer counters run on across segments, so the producer loads the next segment's
 // slabs while the MMAs finish this one, and the epilogue stores a finished segment while
 // the next one's first chunk accumulates in the other TMEM buffer.
-template <class C>
+template <class C, class Work>
 __global__ void __launch_bounds__(C::THREADS, 1)
 split_sk_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmB0,
                 const __grid_constant__ Params P0, const __grid_constant__ CUtensorMap tmA1,
-                const __grid_constant__ CUtensorMap tmB1, const __grid_constant__ Params P1, SkWork W) {
+                const __grid_constant__ CUtensorMap tmB1, const __grid_constant__ Params P1, Work W) {
+    constexpr bool BLOCK = std::is_same<Work, SkBlock>::value;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::STAGES * C::STAGE_BYTES);
@@ -1373,10 +1376,11 @@ split_sk_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant_
             // ---------------- TMA producer ----------------
             prefetch_tmap(&tmA0);
             prefetch_tmap(&tmB0);
-            if (W.tiles1) {
-                prefetch_tmap(&tmA1);
-                prefetch_tmap(&tmB1);
-            }
+            if constexpr (!BLOCK)
+                if (W.tiles1) {
+                    prefetch_tmap(&tmA1);
+                    prefetch_tmap(&tmB1);
+                }
             SkCursor cur = sk_cursor(W, blockIdx.x, gridDim.x);
             SkSeg sg;
             bool ok = true;
@@ -1477,7 +1481,20 @@ split_sk_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant_
             const i64 row = sg.m0 + quarter * 32 + lane;
             if (!ok) continue;
             const i64 cbase = sg.n0 + part * C::EPI_COLS;
-            if (sg.kb0 == 0 && sg.kb1 == (sg.prod ? W.nkb1 : W.nkb0)) split_store_row<C>(P, row, cbase, acc);
+            if constexpr (BLOCK) {
+                // a cut tile's second part is added by the thread that stored its first, which was added
+                // to a zero as sk_zero_kernel's is
+                if (sg.kb0 == 0 && sg.kb1 < sk_slabs(W, 0)) {
+                    const float alpha = float(P.alpha);
+#pragma unroll
+                    for (int j = 0; j < C::EPI_COLS; ++j) acc[j] = alpha * acc[j] + 0.0f;
+                    int lo, hi;
+                    live_columns(P, row, cbase, P.n, lo, hi);
+                    split_store<C::EPI_COLS>(static_cast<float*>(P.c) + row + cbase * P.ldc, P.ldc, 1.0f, 0.0f, acc, lo, hi);
+                    continue;
+                }
+            }
+            if (sg.kb0 == 0 && sg.kb1 == sk_slabs(W, sg.prod)) split_store_row<C>(P, row, cbase, acc);
             else split_add_row<C>(P, row, cbase, acc);
         }
     }
@@ -1931,48 +1948,10 @@ int sk_workers(int dev, int sms, i64& out) {
         return MBG_OK;
     }
     int n = 0;
-    MBG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, split_sk_kernel<C>, C::THREADS, C::SMEM_BYTES));
+    MBG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, split_sk_kernel<C, SkWork>, C::THREADS, C::SMEM_BYTES));
     out = imax(1, imin(i64(n) * sms, sms));
     if (dev >= 0 && dev < 64) cache[dev].store(int(out));
     return MBG_OK;
-}
-
-// Schedule of a persistent split launch over up to G workers (SkWork): whole tiles; when
-// the tiles leave a last wave partly empty (and stream_k allows), stream-K ranges over the
-// last (tiles mod g) + g tiles, with g <= G workers chosen so that every range is at least
-// as long as the longest tile, and only where the busiest worker then finishes clearly
-// sooner than with whole tiles.  G returns the number of workers to launch.
-inline SkWork sk_plan(i64 t0, int n0, i64 t1, int n1, i64& G, bool stream_k) {
-    SkWork W{};
-    W.tiles0 = int(t0);
-    W.tiles1 = int(t1);
-    W.nkb0 = n0;
-    W.nkb1 = t1 ? n1 : n0;
-    const i64 T = t0 + t1;
-    W.dp_tiles = int(T);
-    G = imin(G, T);
-    if (!stream_k || G <= 0 || T % G == 0) return W;
-    auto slab_pos = [&](i64 u) { return u <= t0 ? u * n0 : t0 * n0 + (u - t0) * n1; };
-    const i64 longest = t1 ? imax(n0, n1) : n0;
-    // all tiles in ranges of at least `longest` slabs: as many workers as that allows
-    const i64 total = slab_pos(T);
-    i64 g = imin(G, total / longest);
-    const i64 dp = T > 2 * g ? T - (T % g) - g : 0;
-    const i64 begin = slab_pos(dp);
-    if (g <= 0 || (total - begin) / g < longest) return W;
-    // worth it when the balanced ranges end before whole tiles would: whole tiles take
-    // ceil(T / G) tile times on the busiest worker, the ranges (total - begin) / g slabs
-    // after dp / g whole tiles
-    const double whole = double((T + G - 1) / G) * double(longest);
-    const double ranged = double(dp / g) * double(longest) + double(total - begin) / double(g);
-    // the persistent kernel ran a slab about 5 % slower than tc_gemm_kernel (8192^3 NT, whole
-    // tiles plus a stream-K tail: 4.43 against 4.26 ms): demand a tenth
-    if (1.1 * ranged >= whole) return W;
-    W.dp_tiles = int(dp);
-    W.sk_begin = begin;
-    W.total = total;
-    G = g;
-    return W;
 }
 
 // Persistent launch (split_sk_kernel, config C) of one or two split products; the shared
@@ -1986,7 +1965,7 @@ int launch_sk(const CUtensorMap* ma, const CUtensorMap* mb, Params* P, int nprod
     MBG_CUDA(cudaGetDevice(&dev));
     MBG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     if (!configured_on(configured, dev)) {
-        MBG_CUDA(cudaFuncSetAttribute(split_sk_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        MBG_CUDA(cudaFuncSetAttribute(split_sk_kernel<C, SkWork>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       C::SMEM_BYTES));
         mark_configured(configured, dev);
     }
@@ -2014,8 +1993,42 @@ int launch_sk(const CUtensorMap* ma, const CUtensorMap* mb, Params* P, int nprod
         MBG_CUDA(launch_pdl(sk_zero_kernel<C>, dim3(unsigned(G - 1), SK_ZERO_CTAS), dim3(256), 0, stream(), P[0], P[1], W, int(G)));
         MBG_TRY(check_launch("sk_zero"));
     }
-    MBG_CUDA(launch_pdl(split_sk_kernel<C>, dim3(unsigned(G)), dim3(C::THREADS), C::SMEM_BYTES, stream(), ma[0], mb[0], P[0],
+    MBG_CUDA(launch_pdl(split_sk_kernel<C, SkWork>, dim3(unsigned(G)), dim3(C::THREADS), C::SMEM_BYTES, stream(), ma[0], mb[0], P[0],
                         ma[1], mb[1], P[1], W));
+    return check_launch(name);
+}
+
+// A column block of the pipelined host path, in the schedule of the call over all of C; declined as in
+// launch_sk.
+template <class C>
+int launch_sk_block(const CUtensorMap& ma, const CUtensorMap& mb, Params& P, const char* name, bool* declined) {
+    static_assert(C::TILE_M == BM, "tiles_m counts the tiles");
+    static std::atomic<unsigned> configured{0};  // one bit per device
+    int dev = 0, sms = 148;
+    MBG_CUDA(cudaGetDevice(&dev));
+    MBG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (!configured_on(configured, dev)) {
+        MBG_CUDA(cudaFuncSetAttribute(split_sk_kernel<C, SkBlock>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      C::SMEM_BYTES));
+        mark_configured(configured, dev);
+    }
+    SkBlock B{};
+    B.whole = TileGrid{P.tiles_m, int(cdiv(schedule_columns(P.n), C::TILE_N)), C::TILE_GROUP};
+    B.block = TileGrid{P.tiles_m, P.tiles_n, C::TILE_GROUP};
+    B.tn0 = int(schedule_first_column() / C::TILE_N);
+    const i64 tiles = i64(P.tiles_m) * B.whole.tiles_n;
+    if (P.num_kb <= 0 || tiles > 0x7fffffff) return MBG_ERR_UNSUPPORTED;
+    i64 G = 0;
+    MBG_TRY(sk_workers<C>(dev, sms, G));
+    const i64 ctas = imin(G, i64(P.tiles_m) * P.tiles_n);
+    B.W = sk_plan(tiles, P.num_kb, 0, 0, G, true);
+    B.workers = G;
+    *declined = B.W.total == B.W.sk_begin;
+    if (*declined) return MBG_OK;
+    if (!P.err) P.err = device_error_flag();
+    ProfScope prof(name);
+    MBG_CUDA(launch_pdl(split_sk_kernel<C, SkBlock>, dim3(unsigned(ctas)), dim3(C::THREADS), C::SMEM_BYTES, stream(), ma, mb,
+                        P, ma, mb, P, B));
     return check_launch(name);
 }
 
@@ -2028,7 +2041,7 @@ int prepare_split_kernel(int dev, int sms, bool wide) {
         for (int S = 1; S <= clu::MAX_CTAS; ++S) ck_clusters<C>(dev, S);
     if (wide) {
         i64 workers = 0;
-        MBG_CUDA(cudaFuncSetAttribute(split_sk_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+        MBG_CUDA(cudaFuncSetAttribute(split_sk_kernel<C, SkWork>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
         MBG_TRY(sk_workers<C>(dev, sms, workers));
         cudaFuncAttributes at;
         MBG_CUDA(cudaFuncGetAttributes(&at, sk_zero_kernel<C>));
@@ -2098,7 +2111,8 @@ SplitShape split_shape(const Params& P, int terms, int dev, int sms) {
 // The split product on planes pa (op(A), a_rows rows from pa, planes a_plane_rows apart)
 // and pb (op(B)^T, b_rows rows).  More wide tiles than SMs with a last wave mostly empty (beta = 0,
 // no band, mask or d-vector): split_sk_kernel with a stream-K tail; else the shape that
-// split_shape takes to be fastest.  Sets the B map and P.tiles_n.
+// split_shape takes to be fastest.  Both go by the whole product (ScheduleColumns).  Sets the B map
+// and P.tiles_n.
 int launch_split_product(int terms, const __nv_bfloat16* pa, i64 a_rows, i64 a_plane_rows, const __nv_bfloat16* pb,
                          i64 b_rows, i64 Kp, Params& P) {
     int dev = 0, sms = 148;
@@ -2106,14 +2120,20 @@ int launch_split_product(int terms, const __nv_bfloat16* pa, i64 a_rows, i64 a_p
     MBG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     CUtensorMap ma, mb;
     MBG_TRY(make_map(&ma, pa, false, Kp, a_rows, terms, 64, BM, a_plane_rows));
-    if (i64(P.tiles_m) * cdiv(P.n, 256) > sms && P.beta == 0.0 && !P.tri && P.band == KB_NONE && !P.dvec) {
+    if (i64(P.tiles_m) * cdiv(schedule_columns(P.n), 256) > sms && P.beta == 0.0 && !P.tri && P.band == KB_NONE && !P.dvec) {
         MBG_TRY(make_map(&mb, pb, false, Kp, b_rows, terms, 64, 256));
         P.tiles_n = int(cdiv(P.n, 256));
-        const CUtensorMap mas[2] = {ma, ma}, mbs[2] = {mb, mb};
-        Params Ps[2] = {P, P};
         bool declined = false;
-        const int st = terms == 2 ? launch_sk<CfgBF16x3>(mas, mbs, Ps, 1, true, "tc_gemm_bf16x3", &declined)
-                                  : launch_sk<CfgBF16x6>(mas, mbs, Ps, 1, true, "tc_gemm_bf16x6", &declined);
+        int st = MBG_OK;
+        if (schedule_columns(P.n) != P.n) {
+            st = terms == 2 ? launch_sk_block<CfgBF16x3>(ma, mb, P, "tc_gemm_bf16x3", &declined)
+                            : launch_sk_block<CfgBF16x6>(ma, mb, P, "tc_gemm_bf16x6", &declined);
+        } else {
+            const CUtensorMap mas[2] = {ma, ma}, mbs[2] = {mb, mb};
+            Params Ps[2] = {P, P};
+            st = terms == 2 ? launch_sk<CfgBF16x3>(mas, mbs, Ps, 1, true, "tc_gemm_bf16x3", &declined)
+                            : launch_sk<CfgBF16x6>(mas, mbs, Ps, 1, true, "tc_gemm_bf16x6", &declined);
+        }
         if (st || !declined) return st;
     }
     const SplitShape sh = terms == 2 ? split_shape<CfgBF16x3, CfgBF16x3m>(P, terms, dev, sms)

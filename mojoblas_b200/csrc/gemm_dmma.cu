@@ -360,10 +360,13 @@ int dgemm_dmma(char ta, char tb, i64 m, i64 n, i64 k, double alpha, const double
                const double* b, i64 ldb, double beta, double* c, i64 ldc, int band) {
     ProfScope prof("gemm_dmma_f64");
     const i64 gm = cdiv(m, 128), gn = cdiv(n, 128), ns = schedule_columns(n);
-    if (gm * cdiv(ns, 128) < 2 * 148) {  // under two waves of 128 x 128 tiles: 64 x 64 tiles
+    // under two waves of 128 x 128 tiles: 64 x 64 tiles.  A column block of the pipelined host path
+    // divides its reduction as the call over all of C does; the tile, which changes no sum, goes by
+    // the block (4096^3 on pinned host memory 8.80 ms, 9.26 with the whole product's tiles)
+    const int S = gm * cdiv(ns, 128) < 2 * 148 && band == KB_NONE ? dmma_share(m, ns, k) : 1;
+    if (gm * gn < 2 * 148) {
         const i64 sm = cdiv(m, 64), sn = cdiv(n, 64);
         if (sn > 65535 || sm > 0x7fffffff) return MBG_ERR_UNSUPPORTED;
-        const int S = band == KB_NONE ? dmma_share(m, ns, k) : 1;
         if (S > 1) return launch_dmma_ck(S, is_t(ta), is_t(tb), m, n, k, alpha, a, lda, b, ldb, beta, c, ldc);
         return launch_dmma<Small, 0, 64, 64>(is_t(ta), is_t(tb), dim3((unsigned)sm, (unsigned)sn), m, n, k, alpha,
                                              a, lda, b, ldb, beta, c, ldc, band);

@@ -42,17 +42,18 @@ gemm_f32_kernel(i64 m, i64 n, i64 k, float alpha, const float* __restrict__ A, i
 template <int FT, bool TA, bool TB, bool VA, bool VB>
 __global__ void __launch_bounds__(FNT, FT == 128 ? 2 : 4)
 gemm_f32_ck_kernel(i64 m, i64 n, i64 k, float alpha, const float* __restrict__ A, i64 lda,
-                   const float* __restrict__ B, i64 ldb, float beta, float* __restrict__ C, i64 ldc, unsigned tiles_m) {
+                   const float* __restrict__ B, i64 ldb, float beta, float* __restrict__ C, i64 ldc, unsigned tiles_m,
+                   int unit) {
     extern __shared__ __align__(16) float fsm[];
     pdl_next();
     pdl_wait();
     const unsigned tile = blockIdx.x / clu::size();
     f32_tile<FT, TA, TB, 0, VA, VB, true>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tile % tiles_m, tile / tiles_m,
-                                          fsm);
+                                          fsm, KB_NONE, unit);
 }
 
 template <int FT, bool TA, bool TB, bool VA, bool VB>
-int launch_f32_ck_t(int S, i64 m, i64 n, i64 k, float alpha, const float* a, i64 lda, const float* b, i64 ldb,
+int launch_f32_ck_t(int S, int unit, i64 m, i64 n, i64 k, float alpha, const float* a, i64 lda, const float* b, i64 ldb,
                     float beta, float* c, i64 ldc) {
     constexpr size_t SM = f32_ck_smem<FT>();
     static std::atomic<unsigned> configured{0};  // one bit per device
@@ -66,16 +67,16 @@ int launch_f32_ck_t(int S, i64 m, i64 n, i64 k, float alpha, const float* a, i64
     const unsigned gm = unsigned(cdiv(m, FT));
     const clu::Launch l(gm * unsigned(cdiv(n, FT)) * unsigned(S), S, FNT, SM, stream(), true);
     MBG_CUDA(cudaLaunchKernelEx(&l.cfg, gemm_f32_ck_kernel<FT, TA, TB, VA, VB>, m, n, k, alpha, a, lda, b, ldb, beta,
-                                c, ldc, gm));
+                                c, ldc, gm, unit));
     return check_launch("gemm_f32");
 }
 
 template <int FT>
-int launch_f32_ck(int S, bool ta, bool tb, i64 m, i64 n, i64 k, float alpha, const float* a, i64 lda, const float* b,
-                  i64 ldb, float beta, float* c, i64 ldc) {
+int launch_f32_ck(int S, int unit, bool ta, bool tb, i64 m, i64 n, i64 k, float alpha, const float* a, i64 lda,
+                  const float* b, i64 ldb, float beta, float* c, i64 ldc) {
     const bool va = f32_vec(!ta, a, lda), vb = f32_vec(tb, b, ldb);
 #define CKL(TA_, TB_, VA_, VB_) \
-    return launch_f32_ck_t<FT, TA_, TB_, VA_, VB_>(S, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc)
+    return launch_f32_ck_t<FT, TA_, TB_, VA_, VB_>(S, unit, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc)
     if (!ta && tb) {
         if (va && vb) CKL(false, true, true, true);
         if (va) CKL(false, true, true, false);
@@ -103,26 +104,45 @@ int launch_f32_ck(int S, bool ta, bool tb, i64 m, i64 n, i64 k, float alpha, con
 // with two.)
 struct F32Shape {
     int ft, S;
+    int unit;  // slabs that a CTA's part of the reduction is a multiple of
 };
-inline F32Shape f32_shape(i64 m, i64 n, i64 k, int vec_operands, bool may_share) {
-    F32Shape best{64, 1};
+inline F32Shape f32_shape(i64 m, i64 n, i64 k, int vec_operands, int S_min, int S_max) {
+    F32Shape best{64, S_min, 1};
     double t_best = 0;
     const double scalar = (2 - vec_operands) / 2.0;
     for (int ft = 64; ft <= 128; ft *= 2) {
         const i64 tiles = cdiv(m, ft) * cdiv(n, ft), slabs = cdiv(k, ft == 128 ? Deep<128>::K : Deep<64>::K);
         const double lat = ft == 128 ? 2.75 + 0.4 * scalar : 0.51 + 0.23 * scalar;
         const double rate = ft == 128 ? lat : 0.46 + 0.18 * scalar;
-        for (int S = 1; S <= (may_share ? clu::MAX_CTAS : 1) && S <= slabs; ++S) {
+        for (int S = S_min; S <= S_max && S <= slabs; ++S) {
             const double share = rate * double(cdiv(tiles * S, clu::usable_sms(S)));
             double t = double(cdiv(slabs, S)) * (share > lat ? share : lat) + (S > 1 ? 1.0 + 0.2 * S : 0.0);
             if (ft == 128 || S > 1) t *= 1.1;
             if (t_best == 0 || t < t_best) {
                 t_best = t;
-                best = F32Shape{ft, S};
+                best = F32Shape{ft, S, 1};
             }
         }
     }
     return best;
+}
+
+// The shape of a call.  At sizes that the pipelined host path takes, its column blocks and the call over all
+// of C (on device pointers) have to divide a reduction alike, so the parts go by the whole
+// product and by no alignment (staged copies have leading dimensions of their own).  The tile changes
+// no sum and goes by what runs here: 1024 x 4100 x 4096 on pinned host memory takes 2.33 ms so, and
+// 3.32 with the whole product's 128-tiles, 48 of them in a block.
+inline F32Shape f32_schedule(i64 m, i64 n, i64 k, int vec_operands, bool may_share) {
+    const i64 ns = schedule_columns(n);
+    const bool host_sized = double(m) * double(ns) * double(k) >= double(1ll << 34);
+    auto few = [&](i64 columns) { return cdiv(m, 128) * cdiv(columns, 128) < 2 * 148; };
+    F32Shape sh = few(ns) ? f32_shape(m, ns, k, host_sized ? 2 : vec_operands, 1, may_share ? clu::MAX_CTAS : 1)
+                          : F32Shape{128, 1, 1};
+    if (host_sized && few(n) && (sh.S == 1 || sh.ft == 128)) {
+        const int ft = f32_shape(m, n, k, vec_operands, sh.S, sh.S).ft;
+        sh = F32Shape{ft, sh.S, sh.S > 1 && ft == 64 ? Deep<128>::K / Deep<64>::K : 1};
+    }
+    return sh;
 }
 
 template <int FT, int TRI, bool VA, bool VB>
@@ -226,15 +246,11 @@ int sgemm_f32(char ta, char tb, i64 m, i64 n, i64 k, float alpha, const float* a
         return sgemm_f32(ta, tb, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc, band);
     }
     ProfScope prof("gemm_f32");
-    const i64 gm = cdiv(m, 128), gn = cdiv(n, 128), ns = schedule_columns(n);
-    // (what the pipelined host path takes is scheduled alike whatever the operands' alignment: its
-    // staged copies have leading dimensions of their own)
-    const int vec = double(m) * double(ns) * double(k) >= double(1ll << 34)
-                        ? 2 : int(f32_vec(is_n(ta), a, lda)) + int(f32_vec(is_t(tb), b, ldb));
-    const F32Shape sh = gm * cdiv(ns, 128) >= 2 * 148 ? F32Shape{128, 1} : f32_shape(m, ns, k, vec, band == KB_NONE);
+    const i64 gm = cdiv(m, 128), gn = cdiv(n, 128);
+    const F32Shape sh = f32_schedule(m, n, k, int(f32_vec(is_n(ta), a, lda)) + int(f32_vec(is_t(tb), b, ldb)), band == KB_NONE);
     if (sh.S > 1)
-        return sh.ft == 128 ? launch_f32_ck<128>(sh.S, is_t(ta), is_t(tb), m, n, k, alpha, a, lda, b, ldb, beta, c, ldc)
-                            : launch_f32_ck<64>(sh.S, is_t(ta), is_t(tb), m, n, k, alpha, a, lda, b, ldb, beta, c, ldc);
+        return sh.ft == 128 ? launch_f32_ck<128>(sh.S, sh.unit, is_t(ta), is_t(tb), m, n, k, alpha, a, lda, b, ldb, beta, c, ldc)
+                            : launch_f32_ck<64>(sh.S, sh.unit, is_t(ta), is_t(tb), m, n, k, alpha, a, lda, b, ldb, beta, c, ldc);
     if (sh.ft == 64) {
         const i64 sm = cdiv(m, 64), sn = cdiv(n, 64);
         if (sn > 65535 || sm > 0x7fffffff) return MBG_ERR_UNSUPPORTED;

@@ -102,13 +102,13 @@ __device__ __forceinline__ void f32_stage(float* tile, const float* __restrict__
 // One FT x FT tile (tm, tn) of C := alpha op(A) op(B) + beta C by the whole CTA,
 // staging through `fsm` (f32_smem<FT>() bytes); every copy it issued has landed
 // when it returns.  band (KB_*): one operand triangular, only the tile's slabs run.
-// CK: the CTAs of a cluster share the tile, each taking an equal part of the slabs; each then
+// CK: the CTAs of a cluster share the tile, each taking an equal part of the slabs, by `unit`; each then
 // leaves its sums in its shared memory (f32_ck_smem<FT>() bytes in all) and adds up its share
 // of the columns over the cluster, in the CTAs' order, so results do not depend on scheduling.
 template <int FT, bool TA, bool TB, int TRI, bool VA, bool VB, bool CK = false, class Slab = Deep<FT>>
 __device__ __forceinline__ void f32_tile(i64 m, i64 n, i64 k, float alpha, const float* __restrict__ A, i64 lda,
                                          const float* __restrict__ B, i64 ldb, float beta, float* __restrict__ C,
-                                         i64 ldc, i64 tm, i64 tn, float* fsm, int band = KB_NONE) {
+                                         i64 ldc, i64 tm, i64 tn, float* fsm, int band = KB_NONE, int unit = 1) {
     constexpr int FLD = FTile<FT>::LD, TM = FTile<FT>::TM, FK = Slab::K, FSTAGES = Slab::STAGES;
     float* As = fsm;                               // [stage][k][FLD]
     float* Bs = fsm + size_t(FSTAGES) * FK * FLD;  // [stage][k][FLD]
@@ -132,9 +132,9 @@ __device__ __forceinline__ void f32_tile(i64 m, i64 n, i64 k, float alpha, const
     i64 kt0 = 0, kt1 = (k + FK - 1) / FK;
     if (band != KB_NONE) band_slabs(band, m0, FT, n0, FT, 0, FK, kt1, kt0, kt1);
     if constexpr (CK) {
-        const i64 all = kt1, S = clu::size(), r = clu::rank();
-        kt0 = all * r / S;
-        kt1 = all * (r + 1) / S;
+        const i64 all = (kt1 + unit - 1) / unit, S = clu::size(), r = clu::rank();
+        kt0 = all * r / S * unit;
+        if (r + 1 < S) kt1 = all * (r + 1) / S * unit;
     }
     const i64 nk = kt1 - kt0;
 #pragma unroll

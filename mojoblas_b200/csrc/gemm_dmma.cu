@@ -83,8 +83,7 @@ __global__ void __launch_bounds__(C::THREADS, 1)
 gemm_dmma_kernel(i64 m, i64 n, i64 k, double alpha, const double* __restrict__ A, i64 lda,
                  const double* __restrict__ B, i64 ldb, double beta, double* __restrict__ Cm, i64 ldc, int band) {
     extern __shared__ __align__(16) double dsm[];
-    pdl_next();
-    pdl_wait();
+    pdl_wait();  // (and no pdl_next: launch_pdl)
     // A: TA (k contiguous in memory) -> [m][DKP], else [k][BM + 8]; B: !TB -> [n][DKP], else [k][BN + 8]
     constexpr int LA = TA ? DKP : BM + 8, LB = TB ? BN + 8 : DKP;
     double* As = dsm;

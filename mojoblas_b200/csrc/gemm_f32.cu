@@ -21,8 +21,7 @@ __global__ void __launch_bounds__(FNT, FT == 128 ? 2 : 4)
 gemm_f32_kernel(i64 m, i64 n, i64 k, float alpha, const float* __restrict__ A, i64 lda,
                 const float* __restrict__ B, i64 ldb, float beta, float* __restrict__ C, i64 ldc, int band) {
     extern __shared__ __align__(16) float fsm[];
-    pdl_next();
-    pdl_wait();
+    pdl_wait();  // (and no pdl_next: launch_pdl)
     i64 tm, tn;
     if (TRI == 0) {
         tm = blockIdx.x;
@@ -45,8 +44,7 @@ gemm_f32_ck_kernel(i64 m, i64 n, i64 k, float alpha, const float* __restrict__ A
                    const float* __restrict__ B, i64 ldb, float beta, float* __restrict__ C, i64 ldc, unsigned tiles_m,
                    int unit) {
     extern __shared__ __align__(16) float fsm[];
-    pdl_next();
-    pdl_wait();
+    pdl_wait();  // (and no pdl_next: launch_pdl)
     const unsigned tile = blockIdx.x / clu::size();
     f32_tile<FT, TA, TB, 0, VA, VB, true>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tile % tiles_m, tile / tiles_m,
                                           fsm, KB_NONE, unit);

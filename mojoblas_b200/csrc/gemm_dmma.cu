@@ -330,18 +330,20 @@ int launch_dmma_ck(int S, bool ta, bool tb, i64 m, i64 n, i64 k, double alpha, c
 }
 
 // CTAs per 64 x 64 tile, by the estimated time in microseconds: a 32-deep slab takes 1.7 for a
-// CTA alone on its SM (latency) and 2.3 for the two that fit together (the FP64 pipe's rate);
-// sharing a tile adds 1 + 0.2 S, and has to be worth a tenth.  (Measured around each call, launch
-// included: 300 x 521 x 257 TN 25 us, 17 with three CTAs per tile; 512^3 NT 35, 25 with two and 21
-// with four; 64 x 64 x 1000 TT 58, 17 with eight; 1024 x 1024 x 512 NT 50, 60 with two.)
+// CTA alone on its SM (latency) and 2.3 for the two that fit together (the FP64 pipe's rate); what
+// does not fit waits for a round of its own, whose last CTAs go two to an SM again. Sharing a tile
+// adds 1 + 0.2 S to each round, a further round 1.5 for its start, and has to be worth a tenth.
+// (Measured around each call, launch included: 300 x 521 x 257 TN 25 us, 17 with three CTAs per
+// tile; 512^3 NT 35, 25 with two and 21 with four; 64 x 64 x 1000 TT 58, 17 with eight. Calls in a
+// row: 224 x 1623 x 345 NT 28.7, 26.4 with two and 35.3 with six, which is five rounds.)
 inline int dmma_share(i64 m, i64 n, i64 k) {
     const i64 slabs = cdiv(k, DK), tiles = cdiv(m, 64) * cdiv(n, 64);
     int best = 1;
     double t_best = 0;
     for (int S = 1; S <= clu::MAX_CTAS && S <= slabs; ++S) {
         const i64 per_sm = cdiv(tiles * S, clu::usable_sms(S));
-        const double slab = 2.3 * double(per_sm / 2) + 1.7 * double(per_sm % 2);
-        double t = double(cdiv(slabs, S)) * slab + (S > 1 ? 1.0 + 0.2 * S : 0.0);
+        const double rounds = double(cdiv(per_sm, 2)), slab = per_sm == 1 ? 1.7 : 2.3 * rounds;
+        double t = double(cdiv(slabs, S)) * slab + rounds * (S > 1 ? 1.0 + 0.2 * S : 0.0) + (rounds - 1.0) * 1.5;
         if (S > 1) t *= 1.1;
         if (t_best == 0 || t < t_best) {
             t_best = t;

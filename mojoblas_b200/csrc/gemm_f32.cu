@@ -130,11 +130,15 @@ inline F32Shape f32_shape(i64 m, i64 n, i64 k, int vec_operands, int S_min, int 
 // product and by no alignment (staged copies have leading dimensions of their own).  The tile changes
 // no sum and goes by what runs here: 1024 x 4100 x 4096 on pinned host memory takes 2.33 ms so, and
 // 3.32 with the whole product's 128-tiles, 48 of them in a block.
-inline F32Shape f32_schedule(i64 m, i64 n, i64 k, int vec_operands, bool may_share) {
+//
+// A banded product (trmm) takes 64-tiles when it has few: its tiles' reductions differ in length, and smaller
+// ones fill the chip more evenly (strmm L 2048 x 1024 198 us, 232 on the 128-tiles of f32_shape).
+inline F32Shape f32_schedule(i64 m, i64 n, i64 k, int vec_operands, bool banded) {
     const i64 ns = schedule_columns(n);
     const bool host_sized = double(m) * double(ns) * double(k) >= double(1ll << 34);
     auto few = [&](i64 columns) { return cdiv(m, 128) * cdiv(columns, 128) < 2 * 148; };
-    F32Shape sh = few(ns) ? f32_shape(m, ns, k, host_sized ? 2 : vec_operands, 1, may_share ? clu::MAX_CTAS : 1)
+    if (banded) return F32Shape{few(n) ? 64 : 128, 1, 1};
+    F32Shape sh = few(ns) ? f32_shape(m, ns, k, host_sized ? 2 : vec_operands, 1, clu::MAX_CTAS)
                           : F32Shape{128, 1, 1};
     if (host_sized && few(n) && (sh.S == 1 || sh.ft == 128)) {
         const int ft = f32_shape(m, n, k, vec_operands, sh.S, sh.S).ft;
@@ -245,7 +249,7 @@ int sgemm_f32(char ta, char tb, i64 m, i64 n, i64 k, float alpha, const float* a
     }
     ProfScope prof("gemm_f32");
     const i64 gm = cdiv(m, 128), gn = cdiv(n, 128);
-    const F32Shape sh = f32_schedule(m, n, k, int(f32_vec(is_n(ta), a, lda)) + int(f32_vec(is_t(tb), b, ldb)), band == KB_NONE);
+    const F32Shape sh = f32_schedule(m, n, k, int(f32_vec(is_n(ta), a, lda)) + int(f32_vec(is_t(tb), b, ldb)), band != KB_NONE);
     if (sh.S > 1)
         return sh.ft == 128 ? launch_f32_ck<128>(sh.S, sh.unit, is_t(ta), is_t(tb), m, n, k, alpha, a, lda, b, ldb, beta, c, ldc)
                             : launch_f32_ck<64>(sh.S, sh.unit, is_t(ta), is_t(tb), m, n, k, alpha, a, lda, b, ldb, beta, c, ldc);

@@ -16,7 +16,7 @@ namespace {
 
 using namespace f32t;
 
-template <int FT, bool TA, bool TB, int TRI, bool VA, bool VB>
+template <int FT, bool TA, bool TB, int TRI, bool VA, bool VB, class Slab>
 __global__ void __launch_bounds__(FNT, FT == 128 ? 2 : 4)
 gemm_f32_kernel(i64 m, i64 n, i64 k, float alpha, const float* __restrict__ A, i64 lda,
                 const float* __restrict__ B, i64 ldb, float beta, float* __restrict__ C, i64 ldc, int band) {
@@ -32,7 +32,7 @@ gemm_f32_kernel(i64 m, i64 n, i64 k, float alpha, const float* __restrict__ A, i
         f32_tri_tile(blockIdx.x, ti, tj);
         if (TRI == 1) { tm = ti; tn = tj; } else { tm = tj; tn = ti; }
     }
-    f32_tile<FT, TA, TB, TRI, VA, VB>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tm, tn, fsm, band);
+    f32_tile<FT, TA, TB, TRI, VA, VB, false, Slab>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tm, tn, fsm, band);
 }
 
 
@@ -147,27 +147,27 @@ inline F32Shape f32_schedule(i64 m, i64 n, i64 k, int vec_operands, bool banded)
     return sh;
 }
 
-template <int FT, int TRI, bool VA, bool VB>
-int launch_f32_v(bool ta, bool tb, dim3 grid, i64 m, i64 n, i64 k, float alpha, const float* a, i64 lda,
-                 const float* b, i64 ldb, float beta, float* c, i64 ldc, int band) {
-    constexpr size_t SM = f32_smem<FT>();
+template <int FT, int TRI, bool VA, bool VB, class Slab>
+int launch_f32_slab(bool ta, bool tb, dim3 grid, i64 m, i64 n, i64 k, float alpha, const float* a, i64 lda,
+                    const float* b, i64 ldb, float beta, float* c, i64 ldc, int band) {
+    constexpr size_t SM = f32_smem<FT, Slab>();
     static std::atomic<unsigned> configured{0};  // one bit per device: more than 48 KB of shared memory needs an opt-in
     int dev = 0;
     MBG_CUDA(cudaGetDevice(&dev));
     if (!configured_on(configured, dev)) {
-        MBG_CUDA(cudaFuncSetAttribute(gemm_f32_kernel<FT, false, false, TRI, VA, VB>,
+        MBG_CUDA(cudaFuncSetAttribute(gemm_f32_kernel<FT, false, false, TRI, VA, VB, Slab>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM));
-        MBG_CUDA(cudaFuncSetAttribute(gemm_f32_kernel<FT, false, true, TRI, VA, VB>,
+        MBG_CUDA(cudaFuncSetAttribute(gemm_f32_kernel<FT, false, true, TRI, VA, VB, Slab>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM));
-        MBG_CUDA(cudaFuncSetAttribute(gemm_f32_kernel<FT, true, false, TRI, VA, VB>,
+        MBG_CUDA(cudaFuncSetAttribute(gemm_f32_kernel<FT, true, false, TRI, VA, VB, Slab>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM));
-        MBG_CUDA(cudaFuncSetAttribute(gemm_f32_kernel<FT, true, true, TRI, VA, VB>,
+        MBG_CUDA(cudaFuncSetAttribute(gemm_f32_kernel<FT, true, true, TRI, VA, VB, Slab>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM));
         mark_configured(configured, dev);
     }
     cudaStream_t s = stream();
-#define F32(TA_, TB_)                                                                                             \
-    MBG_CUDA(launch_pdl(gemm_f32_kernel<FT, TA_, TB_, TRI, VA, VB>, grid, dim3(FNT), SM, s, m, n, k, alpha, a, lda, b, \
+#define F32(TA_, TB_)                                                                                                   \
+    MBG_CUDA(launch_pdl(gemm_f32_kernel<FT, TA_, TB_, TRI, VA, VB, Slab>, grid, dim3(FNT), SM, s, m, n, k, alpha, a, lda, b, \
                         ldb, beta, c, ldc, band))
     if (!ta && !tb) F32(false, false);
     else if (!ta && tb) F32(false, true);
@@ -177,6 +177,19 @@ int launch_f32_v(bool ta, bool tb, dim3 grid, i64 m, i64 n, i64 k, float alpha, 
     return check_launch("gemm_f32");
 }
 
+// 128-tiles take deep slabs where an operand takes 16-byte copies (element by element, the 32 copies of
+// a slab per thread and operand spill: 4096^3 NT with odd leading dimensions 3.12 ms in slabs of 16, 3.73 in
+// slabs of 32) and where the padding of k costs less than they save, a tenth with both operands so
+// (4096 x 4096 x 40: 55 us, 62 as two slabs of 32; x 144 both 118) and a fiftieth with one (4096^3 NN with
+// odd leading dimensions 3.02 and 2.98 ms; 4096 x 4096 x 144 139 and 149 us).
+template <int FT, int TRI, bool VA, bool VB>
+int launch_f32_v(bool ta, bool tb, dim3 grid, i64 m, i64 n, i64 k, float alpha, const float* a, i64 lda,
+                 const float* b, i64 ldb, float beta, float* c, i64 ldc, int band) {
+    if constexpr (FT == 128 && (VA || VB))
+        if ((VA && VB ? 92 : 97) * cdiv(k, Deep<128>::K) * Deep<128>::K <= 100 * cdiv(k, Shallow::K) * Shallow::K)
+            return launch_f32_slab<FT, TRI, VA, VB, Deep<128>>(ta, tb, grid, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc, band);
+    return launch_f32_slab<FT, TRI, VA, VB, Shallow>(ta, tb, grid, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc, band);
+}
 
 template <int FT, int TRI>
 int launch_f32(bool ta, bool tb, dim3 grid, i64 m, i64 n, i64 k, float alpha, const float* a, i64 lda,

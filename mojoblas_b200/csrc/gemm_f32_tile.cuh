@@ -5,8 +5,8 @@
 // block per thread, rows tx*4+{0..3} and 64+tx*4+{0..3}, columns likewise from
 // ty; FT = 64: 4 x 4), one FMA per product (two products per fma.rn.f32x2
 // instruction), each element's sum running over k in ascending order as in the
-// reference's column loops.  K advances in slabs (32 deep in two stages for 128-tiles, 16 in
-// three for 64-tiles) through a cp.async pipeline straight into shared memory: an operand
+// reference's column loops (CK: over each CTA's part of k, then over the parts).  K advances in slabs
+// (32 deep in two stages or 16 in three) through a cp.async pipeline straight into shared memory: an operand
 // contiguous along m (n), 16-byte aligned with ld % 4 == 0, is copied 16 bytes
 // at a time, any other operand element by element into the same k-major tiles
 // (rows padded to FT + 4 floats).  beta == 0 writes C without reading it,
@@ -26,9 +26,10 @@ template <int FT> struct FTile {
     static constexpr int TM = FT / 16;    // rows (and columns) per thread: 8 or 4
 };
 // Slab depth and stages.  Between slabs the FP32 pipe waits for a barrier and first loads, so 128-tiles
-// take deep ones (sgemm NT 4096^3: 16 x 3 stages 2.62 ms, 16 x 4 2.52, 24 x 3 2.54, 8 x 4 2.48, 32 x 3
-// 2.37, 32 x 2 2.36); 64-tiles keep short reductions divisible among CTAs, and grouped plans
-// (Shallow) theirs from being padded (4096 problems of 16..512 on 32 x 2: 1.69 ms against 1.62).
+// take deep ones where that pays (launch_f32_v; sgemm NT 4096^3: 16 x 3 stages 2.62 ms, 16 x 4
+// 2.52, 24 x 3 2.54, 8 x 4 2.48, 32 x 3 2.37, 32 x 2 2.36); 64-tiles keep short reductions
+// divisible among CTAs, and grouped plans theirs from being padded (4096 problems of 16..512 on
+// 32 x 2: 1.69 ms against 1.62).
 template <int FT> struct Deep {
     static constexpr int K = FT == 128 ? 32 : 16, STAGES = FT == 128 ? 2 : 3;
 };

@@ -286,7 +286,6 @@ __device__ __forceinline__ void tc_gemm_tile(const CUtensorMap& tmA, const CUten
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    pdl_next();
     pdl_wait();
 
     if (warp == 0) {
@@ -800,7 +799,6 @@ ozaki_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    pdl_next();
     pdl_wait();
     const int total = C::NPASS * nkb;
 
@@ -1099,7 +1097,6 @@ ozaki_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     const uint32_t leader_tempty = peer_addr(tempty, 0);
-    pdl_next();
     pdl_wait();
 
     if (warp == 0) {
@@ -1368,7 +1365,6 @@ split_sk_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    pdl_next();
     pdl_wait();
 
     if (warp == 0) {

@@ -22,28 +22,26 @@ def test_cluster_barrier_has_converged_warps():
     assert "__syncwarp();" in bodies[0].split("barrier.cluster")[0]
 
 
-def test_next_kernel_is_let_in_after_the_tmem_allocation():
-    """A dependent kernel's blocks may start once every block has called pdl_next().  Before this
-    kernel has its TMEM they could take it, and then wait for this kernel, which waits for them."""
+def test_kernels_with_tmem_let_no_kernel_in():
+    """A dependent kernel's blocks may start once every block has called pdl_next().  They could take the TMEM
+    that this kernel is yet to allocate, and then wait for this kernel, which waits for them."""
     seen = 0
     for name, text in SOURCES.items():
         for head, body in functions(text):
-            if "tmem_alloc" in body and "pdl_next" in body:
-                alloc = body.rindex("tmem_alloc")
-                ready = re.search(r"__syncthreads\(\)|clu::sync_all\(\)", body[alloc:])
-                assert ready and body.index("pdl_next") > alloc + ready.start(), (name, head)
+            if "tmem_alloc" in body and "pdl_wait" in body:
+                assert "pdl_next" not in body, (name, head)
                 seen += 1
     assert seen == 4
 
 
 def test_kernels_of_a_chain_wait_on_every_path():
-    """A kernel that lets the next one in takes part in a chain of dependent launches, whose order holds
-    because each waits for the one before: pdl_wait() follows pdl_next(), and a block that
-    leaves before that has waited too."""
+    """A kernel that lets the next one in, or waits for the one before, takes part in a chain of dependent
+    launches, whose order holds because each waits: pdl_wait() follows pdl_next(), and a block
+    that leaves before the kernel's wait has waited too."""
     for name, text in SOURCES.items():
         for head, body in functions(text):
-            if "pdl_next();" not in body or "pdl_wait() {" in head:
-                continue
-            assert re.search(r"pdl_next\(\);\s*pdl_wait\(\);", body), (name, head)
-            before = body[:body.index("pdl_next();")]
-            assert all(re.search(r"pdl_wait\(\);\s*$", part) for part in before.split("return;")[:-1]), (name, head)
+            if "pdl_next();" in body:
+                assert re.search(r"pdl_next\(\);\s*pdl_wait\(\);", body), (name, head)
+            if "pdl_wait();" in body:
+                before = body[:body.rindex("pdl_wait();")]
+                assert all(re.search(r"pdl_wait\(\);\s*$", part) for part in before.split("return;")[:-1]), (name, head)

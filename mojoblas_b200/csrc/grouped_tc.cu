@@ -22,6 +22,8 @@
 //                step into a TMEM accumulator of 128 x BN fp32 (BN = 64 or 128
 //                per problem), restarted every 128 k (the tensor core's fp32
 //                accumulation truncates) into the other of two buffers;
+//   warps 17..19 prefetch the slabs six (BF16x3: eight) ahead of the products into L2: a producer's
+//                registers hold one slab of loads, too little in flight to cover HBM;
 //   warps 20..27 epilogue: add each 128-k chunk into fp32 registers with
 //                round-to-nearest, then alpha / beta and the column-major store;
 //                the other TMEM buffer lets the next tile's products run meanwhile.
@@ -33,10 +35,13 @@
 // Bound: shared memory, which carries per 32-deep slab of a 128 x 128 tile the products' operand
 // reads (60 KB with A from the collector), the terms' stores (48 KB) and the loads' lines
 // (40 KB), and the start and end of tiles of five slabs on average.  4096 problems (m, n, k
-// log-uniform 16..512, NN, BF16x6): 0.567 ms, of which 0.36 ms remain without loads, splits and
-// stores of C.  Copying each slab to shared memory first (4-byte cp.async, one slab ahead) and
-// splitting from there took 0.697 ms: about 50 cycles for each copy instruction of eight
-// producer warps, and branches around each column of the epilogue's stores.
+// log-uniform 16..512, NN, BF16x6): 0.534 ms (0.567 without the prefetch), of which 0.36 ms remain
+// without loads, splits and stores of C.  Copying each slab to shared memory first (4-byte cp.async,
+// one slab ahead) and splitting from there took 0.697 ms: about 50 cycles for each copy instruction of
+// eight producer warps, and branches around each column of the epilogue's stores.  For many small
+// aligned problems, which HBM bounds, the prefetch is what makes up for its 16-byte copies: 3000 of
+// 96 x 96 x 96, TN, BF16x3 94 us with them, 148 with neither and 91 with the prefetch and the loads of
+// aligned pairs.
 #include "mbg_internal.cuh"
 #include "gemm_f32_tile.cuh"
 #include "schedule.cuh"
@@ -59,11 +64,12 @@ constexpr int GCHUNK = 4;      // slabs per TMEM accumulation chunk
 constexpr int GGROUPS = 2;                // producer groups, taking slabs in turn
 constexpr int GGROUP_WARPS = 8;           // 4 for op(A), 4 for op(B)^T
 constexpr int GPROD_WARPS = GGROUPS * GGROUP_WARPS;
-constexpr int GMMA_WARP = GPROD_WARPS;    // and three idle warps: registers are dealt per four warps
+constexpr int GMMA_WARP = GPROD_WARPS;
+constexpr int GPREFETCH_WARPS = 3;        // with the MMA warp: registers are dealt per four warps
 constexpr int GEPI_WARP0 = GMMA_WARP + 4;
 constexpr int GEPI_WARPS = 8;
 constexpr int GTHREADS = 32 * (GEPI_WARP0 + GEPI_WARPS);
-// 896 threads start with 72 registers: 64512 = 512 x 64 (producers) + 128 x 24 + 256 x 112 (epilogue)
+// 896 threads start with 72 registers: 64512 = 512 x 72 (producers) + 128 x 24 + 256 x 96 (epilogue)
 constexpr int GREGS_PROD = 72, GREGS_MMA = 24, GREGS_EPI = 96;
 static_assert(32 * GPROD_WARPS * GREGS_PROD + 128 * GREGS_MMA + 32 * GEPI_WARPS * GREGS_EPI <= GTHREADS * 72,
               "the register split must fit what the CTA was launched with");
@@ -76,6 +82,7 @@ struct GCfg {
     static constexpr int STAGES = TERMS == 3 ? 4 : 6;  // split planes in flight to the MMA warp
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
     static constexpr int NPROD = TERMS * (TERMS + 1) / 2;
+    static constexpr int AHEAD = TERMS == 3 ? 6 : 8;  // slabs prefetched ahead of the products
     static_assert(SMEM_BYTES <= 232448, "shared memory budget");
 };
 
@@ -89,22 +96,30 @@ struct __align__(16) TcTile {
     int nkb, last;   // k slabs (0 when alpha == 0 or k == 0: C := beta C only), elements of the last
     int rows, cols;  // of the tile inside the problem
     int bn;          // tile columns: 64 or 128
-    int kcontig;     // bit 0: op(A)'s k is the contiguous dimension, bit 1: op(B)'s
+    int kcontig;     // bit 0: op(A)'s k is the contiguous dimension, bit 1: op(B)'s; bits 2, 3: and a pair of k is
+                     // 8-byte aligned in every row
     float alpha, beta;
 };
 
 // A warp's 32 rows (rw0 ..) of a k slab, `left` deep from p on, as 16 k-adjacent pairs per lane: pair i
 // is k (2 i, 2 i + 1) of row rw0 + lane, or, KC (k contiguous), k (2 q, 2 q + 1) of row
 // rw0 + 2 i + h with (h, q) = (lane / 16, lane % 16), so that a load covers two rows of 128 bytes.
-// Zeros past the operand's rows and past the slab's end.
+// Zeros past the operand's rows and past the slab's end.  even: pairs are 8-byte aligned.
 template <bool KC>
 __device__ __forceinline__ void load_pairs(float (&v)[32], const float* __restrict__ p, i64 ld, int rw0, int rows,
-                                           int left, int lane) {
+                                           int left, int lane, bool even = false) {
     if (KC) {
         const int h = lane >> 4, k = 2 * (lane & 15);
         const float* q = p + i64(rw0 + h) * ld + k;
         const bool on0 = k < left, on1 = k + 1 < left;
-        if (rw0 + 32 <= rows && left == GBK) {
+        if (rw0 + 32 <= rows && left == GBK && even) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i, q += 2 * ld) {
+                const float2 w = __ldg(reinterpret_cast<const float2*>(q));
+                v[2 * i] = w.x;
+                v[2 * i + 1] = w.y;
+            }
+        } else if (rw0 + 32 <= rows && left == GBK) {
 #pragma unroll
             for (int i = 0; i < 16; ++i, q += 2 * ld) {
                 v[2 * i] = __ldg(q);
@@ -183,6 +198,26 @@ __device__ __forceinline__ void split_store(const float (&v)[32], uint8_t* plane
     }
 }
 
+// Starts the fetch of a tile's k slab kb into L2, a warp's work: a row or a k per lane.
+__device__ __forceinline__ void prefetch_slab(const TcTile* d, int kb, int nkb, int lane) {
+    const int left = k_left(nkb, d->last, kb, GBK);
+#pragma unroll 1
+    for (int side = 0; side < 2; ++side) {
+        const i64 ld = side ? d->ldb : d->lda;
+        const int rows = side ? d->cols : d->rows;
+        const float* q = side ? d->b : d->a;
+        if ((d->kcontig >> side) & 1) {
+            q += i64(kb) * GBK + lane * ld;
+#pragma unroll 1
+            for (int r = lane; r < rows; r += 32, q += 32 * ld) asm volatile("prefetch.global.L2 [%0];" ::"l"(q));
+        } else if (lane < left) {
+            q += (i64(kb) * GBK + lane) * ld;
+#pragma unroll 1
+            for (int r = 0; r < rows; r += 32, q += 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(q));
+        }
+    }
+}
+
 __device__ __forceinline__ void st_if(float* p, float v, bool on) {  // no branch per element
     asm volatile("{ .reg .pred q; setp.ne.s32 q, %2, 0; @q st.global.f32 [%0], %1; }" ::"l"(p), "f"(v), "r"(int(on))
                  : "memory");
@@ -199,9 +234,11 @@ grouped_tc_kernel(const TcTile* __restrict__ tiles, int ntiles, int* err) {
     uint64_t* tfull = empty + C::STAGES;  // [2]
     uint64_t* tempty = tfull + 2;       // [2]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
+    volatile int* const slabs_done = reinterpret_cast<volatile int*>(tmem_slot + 1);  // slabs the MMA warp has issued
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
+        *slabs_done = 0;
         for (int s = 0; s < C::STAGES; ++s) {
             mbar_init(&full[s], GGROUP_WARPS);
             mbar_init(&empty[s], 1);
@@ -242,7 +279,7 @@ grouped_tc_kernel(const TcTile* __restrict__ tiles, int ntiles, int* err) {
                 o.last = d->last;
                 o.rows = isA ? d->rows : d->cols;
                 o.used = isA ? BM : d->bn;
-                o.kc = (d->kcontig >> (isA ? 0 : 1)) & 1;
+                o.kc = (d->kcontig >> (isA ? 0 : 1)) & 5;
             }
             return o;
         };
@@ -259,7 +296,7 @@ grouped_tc_kernel(const TcTile* __restrict__ tiles, int ntiles, int* err) {
                     float v[32];
                     const int left = k_left(o.nkb, o.last, kb, GBK);
                     if (o.kc) {
-                        load_pairs<true>(v, p, o.ld, rw0, o.rows, left, lane);
+                        load_pairs<true>(v, p, o.ld, rw0, o.rows, left, lane, o.kc & 4);
                         if (!mbar_wait(&empty[s], (use & 1) ^ 1, err, 31)) { ok = false; break; }
                         split_store<TERMS, true>(v, plane0, plane_bytes, rw0, lane);
                     } else {
@@ -322,11 +359,29 @@ grouped_tc_kernel(const TcTile* __restrict__ tiles, int ntiles, int* err) {
                         }
                     }
                     umma_commit(&empty[s]);
+                    *slabs_done = it + 1;
                     if (kin == GCHUNK - 1 || kb == nkb - 1) {
                         umma_commit(&tfull[buf]);
                         ++ch;
                     }
                 }
+            }
+            *slabs_done = 0x7fffffff;  // also after an expired wait
+        } else if (warp > GMMA_WARP) {
+            // ---------------- prefetch: every third slab each ----------------
+            int first = 0, done = 0, mine = warp - GMMA_WARP - 1;  // slabs before the tile; this warp's next one
+            for (int t = blockIdx.x; t < ntiles && done < 0x7fffffff; t += gridDim.x) {
+                const int nkb = tiles[t].nkb;
+                for (; mine < first + nkb; mine += GPREFETCH_WARPS) {
+                    for (int tries = 0; done < mine - C::AHEAD && tries < 100000; ++tries) {
+                        done = *slabs_done;
+                        if (done < mine - C::AHEAD) __nanosleep(50);
+                    }
+                    if (done < mine - C::AHEAD) done = 0x7fffffff;  // no progress: only the prefetches end
+                    if (done == 0x7fffffff) break;
+                    if (mine >= done + GGROUPS) prefetch_slab(tiles + t, mine - first, nkb, lane);
+                }
+                first += nkb;
             }
         }
         __syncwarp();
@@ -422,13 +477,15 @@ int grouped_tc_build(int terms, int count, const mbg_sgemm_problem* probs, Group
         d.nkb = int(slabs.n);
         d.last = slabs.last;
         d.bn = bn;
-        d.kcontig = (ta ? 1 : 0) | (tb ? 0 : 2);
         d.alpha = q.alpha; d.beta = q.beta;
         for (i64 n0 = 0; n0 < q.n; n0 += bn)
             for (i64 m0 = 0; m0 < q.m; m0 += BM) {
                 d.a = q.a + (d.nkb ? (ta ? m0 * q.lda : m0) : 0);
                 d.b = q.b + (d.nkb ? (tb ? n0 : n0 * q.ldb) : 0);
                 d.c = q.c + m0 + n0 * q.ldc;
+                d.kcontig = (ta ? 1 : 0) | (tb ? 0 : 2);
+                if (ta && q.lda % 2 == 0 && reinterpret_cast<uintptr_t>(d.a) % 8 == 0) d.kcontig |= 4;
+                if (!tb && q.ldb % 2 == 0 && reinterpret_cast<uintptr_t>(d.b) % 8 == 0) d.kcontig |= 8;
                 d.rows = int(imin(i64(BM), q.m - m0));
                 d.cols = int(imin(i64(bn), q.n - n0));
                 t.push_back(d);

@@ -51,6 +51,20 @@ MBG_HD i64 tile_index(const TileGrid& q, int tm, int tn) {
     return i64(first_m) * q.tiles_n + i64(tn) * gsize + (tm - first_m);
 }
 
+// Tiles of bm x bn, tiles_m x ceil(n / bn) of them, that a triangle mask keeps (tri: 0 all, 1 those not
+// strictly above the diagonal, 2 not strictly below), counted row by row: every product asks, ahead
+// of its launch.
+inline i64 kept_tiles(int tri, i64 tiles_m, i64 n, int bm, int bn) {
+    const i64 all = (n + bn - 1) / bn;
+    if (!tri) return tiles_m * all;
+    i64 kept = 0;
+    for (i64 tm = 0; tm < tiles_m; ++tm) {
+        const i64 row = tri == 1 ? ((tm + 1) * bm + bn - 1) / bn : all - tm * bm / bn;
+        kept += row > all ? all : row < 0 ? 0 : row;
+    }
+    return kept;
+}
+
 // Work of one persistent split launch (split_sk_kernel): one or two products (the second:
 // the gemm adjoint's other gradient).  Tiles are numbered product 0's first, then product 1's.
 //   whole tiles:  the first dp_tiles tiles, worker (CTA) c taking tiles c, c + G, ...

@@ -2056,21 +2056,6 @@ int prepare_split_kernels() {
     return prepare_split_kernel<CfgBF16x6n>(dev, sms, false);
 }
 
-// Tiles of 128 x bn that the triangle mask keeps.
-inline i64 live_tiles(const Params& P, i64 n, int bn) {
-    const i64 tn_all = cdiv(n, bn);
-    if (!P.tri) return i64(P.tiles_m) * tn_all;
-    i64 live = 0;
-    for (i64 tm = 0; tm < P.tiles_m; ++tm)
-        for (i64 tn = 0; tn < tn_all; ++tn) {
-            const i64 m0 = tm * BM, n0 = tn * bn;
-            if (P.tri == 1 && m0 + BM <= n0) continue;
-            if (P.tri == 2 && m0 > n0 + bn - 1) continue;
-            ++live;
-        }
-    return live;
-}
-
 // Tile width and CTAs per tile of a split product, by the estimated time in microseconds of its
 // waves: a CTA's start and end, and its 32-deep slabs, which take longer the more of the chip
 // reads planes at once.  Measured for six products (slabs of 128 x 256 / 128 / 64 tiles): 0.76,
@@ -2087,7 +2072,7 @@ SplitShape split_shape(const Params& P, i64 n, int S_min, int S_max, int terms, 
     SplitShape best{256, S_min};
     double t_best = 0;
     for (int bn = 256; bn >= 64; bn /= 2) {
-        const i64 tiles = imax(1, live_tiles(P, n, bn));
+        const i64 tiles = imax(1, kept_tiles(P.tri, P.tiles_m, n, BM, bn));
         for (int S = S_min; S <= (bn >= 128 && P.band == KB_NONE && !P.dvec ? S_max : 1) && S <= P.num_kb; ++S) {
             const i64 room = S == 1 ? sms : bn == 256 ? ck_clusters<Wide>(dev, S) : ck_clusters<Mid>(dev, S);
             if (room <= 0) continue;

@@ -33,6 +33,7 @@ void place(int tiles_m, int tiles_n, int group, int t, int* tm, int* tn) {
     const TileAt at = tile_at(TileGrid{tiles_m, tiles_n, group}, t);
     *tm = at.tm; *tn = at.tn;
 }
+i64 kept(int tri, i64 tiles_m, i64 n, int bm, int bn) { return kept_tiles(tri, tiles_m, n, bm, bn); }
 // The cut of tile t of the column block of `cols` tile columns from tn0 on.
 int block_cut(int tiles_m, int tiles_n, int group, int nkb, i64 sms, int tn0, int cols, int t) {
     SkBlock B{};
@@ -61,6 +62,8 @@ def sched(tmp_path_factory):
     lib.slab_count.restype = C.c_int64
     lib.slab_count.argtypes = [C.c_int64, C.c_int]
     lib.slab_left.argtypes = [C.c_int64, C.c_int, C.c_int64]
+    lib.kept.restype = C.c_int64
+    lib.kept.argtypes = [C.c_int, C.c_int64, C.c_int64, C.c_int, C.c_int]
     lib.plan.restype = lib.range_begin.restype = C.c_int64
     lib.plan.argtypes = [C.c_int, C.c_int, C.c_int, C.c_int64, C.POINTER(C.c_int64)]
     lib.range_begin.argtypes = [C.c_int64] * 4
@@ -108,3 +111,25 @@ def test_column_blocks_cut_tiles_as_the_whole_schedule(sched, tiles_m, tiles_n, 
             got[tm.value, tn0 + tn.value] = sched.block_cut(tiles_m, tiles_n, group, nkb, sms, tn0, cols, t)
         tn0 += cols
     assert got == want
+
+
+@pytest.mark.parametrize("bn", [64, 128, 256])
+@pytest.mark.parametrize("tri", [0, 1, 2])
+def test_tiles_that_a_mask_keeps(sched, tri, bn):
+    for m, n in ((1, 1), (128, 128), (129, 130), (700, 700), (1025, 513), (513, 1025), (3000, 3000), (4096, 100)):
+        tiles_m = -(-m // 128)
+        want = sum(not (tri == 1 and 128 * tm + 128 <= bn * tn or tri == 2 and 128 * tm > bn * tn + bn - 1)
+                   for tm in range(tiles_m) for tn in range(-(-n // bn)))
+        assert sched.kept(tri, tiles_m, n, 128, bn) == want, (m, n)
+
+
+def test_counting_kept_tiles_is_quick(sched):
+    """On the launch path of every masked product: 65536 x 65536 has half a million tiles of 128 x 64."""
+    import time
+    best = float("inf")
+    for _ in range(5):
+        start = time.perf_counter()
+        for bn in (64, 128, 256):
+            sched.kept(1, 512, 65536, 128, bn)
+        best = min(best, time.perf_counter() - start)
+    assert best < 1e-4

@@ -100,14 +100,11 @@ struct Cfg {
 
 using CfgBF16x3 = Cfg<false, 2, 256, 64, 4, 8, 4>;
 using CfgBF16x6 = Cfg<false, 3, 256, 64, 3, 8, 4>;
-// 128 x 64 tiles for products too small to give a quarter of the SMs a 128 x 256 tile (the
-// trsm recursion's 512-row blocks: 8 CTAs of the wide tile against 32 of these)
-using CfgBF16x3n = Cfg<false, 2, 64, 64, 8, 8, 4>;
-using CfgBF16x6n = Cfg<false, 3, 64, 64, 6, 8, 4>;
-// 128 x 128 tiles for products that give fewer CTAs than SMs with 128 x 256 tiles: twice the
-// CTAs, so a last partial wave idles less of the GPU (the gemm adjoint's two products)
+// 128 x 128 and 128 x 64 tiles, for products that fill the chip better with more of them (split_shape)
 using CfgBF16x3m = Cfg<false, 2, 128, 64, 6, 8, 4>;
 using CfgBF16x6m = Cfg<false, 3, 128, 64, 4, 8, 4>;
+using CfgBF16x3n = Cfg<false, 2, 64, 64, 8, 8, 4>;
+using CfgBF16x6n = Cfg<false, 3, 64, 64, 6, 8, 4>;
 
 struct Params {
     i64 m, n;
@@ -2031,11 +2028,11 @@ int launch_sk_block(const CUtensorMap& ma, const CUtensorMap& mb, Params& P, con
 // Everything that launch_split_product may launch, loaded and configured ahead of its first use
 // (loading maps code on the device).
 template <class C>
-int prepare_split_kernel(int dev, int sms, bool wide) {
+int prepare_split_kernel(int dev, int sms) {
     MBG_CUDA(cudaFuncSetAttribute(tc_gemm_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
-    if (C::BN >= 128)
-        for (int S = 1; S <= clu::MAX_CTAS; ++S) ck_clusters<C>(dev, S);
-    if (wide) {
+    if constexpr (C::BN >= 128)
+        for (int S = 2; S <= clu::MAX_CTAS; ++S) ck_clusters<C>(dev, S);
+    if constexpr (C::BN == 256) {
         i64 workers = 0;
         MBG_CUDA(cudaFuncSetAttribute(split_sk_kernel<C, SkWork>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
         MBG_TRY(sk_workers<C>(dev, sms, workers));
@@ -2048,12 +2045,12 @@ int prepare_split_kernels() {
     int dev = 0, sms = 148;
     MBG_CUDA(cudaGetDevice(&dev));
     MBG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    MBG_TRY(prepare_split_kernel<CfgBF16x3>(dev, sms, true));
-    MBG_TRY(prepare_split_kernel<CfgBF16x6>(dev, sms, true));
-    MBG_TRY(prepare_split_kernel<CfgBF16x3m>(dev, sms, false));
-    MBG_TRY(prepare_split_kernel<CfgBF16x6m>(dev, sms, false));
-    MBG_TRY(prepare_split_kernel<CfgBF16x3n>(dev, sms, false));
-    return prepare_split_kernel<CfgBF16x6n>(dev, sms, false);
+    MBG_TRY(prepare_split_kernel<CfgBF16x3>(dev, sms));
+    MBG_TRY(prepare_split_kernel<CfgBF16x6>(dev, sms));
+    MBG_TRY(prepare_split_kernel<CfgBF16x3m>(dev, sms));
+    MBG_TRY(prepare_split_kernel<CfgBF16x6m>(dev, sms));
+    MBG_TRY(prepare_split_kernel<CfgBF16x3n>(dev, sms));
+    return prepare_split_kernel<CfgBF16x6n>(dev, sms);
 }
 
 // Tile width and CTAs per tile of a split product, by the estimated time in microseconds of its

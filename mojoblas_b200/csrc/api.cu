@@ -138,9 +138,10 @@ static int gemm_compute(int mode, int slices, char ta, char tb, i64 m, i64 n, i6
 
 // Large gemm with host operands: the host <-> device copies overlap the
 // arithmetic.  C is cut into column blocks: GEMM_PIPE_BLOCKS blocks of equal
-// width (multiples of 256 columns, so every tile of C is the same as in one call
-// over all of C), the last of them halved down to 256 columns so that little
-// arithmetic and little copying is left after op(B)'s last columns land.  A copy
+// width (multiples of 256 columns, so that no tile of C straddles two; every
+// element's sum is divided as in one call over all of C, ScheduleColumns), the last
+// of them halved down to 256 columns so that little arithmetic and little copying is
+// left after op(B)'s last columns land.  A copy
 // stream brings op(A) over first and then, block by block, the columns of op(B)
 // (and of C when beta != 0); the library's stream computes each block as soon as
 // its operands have landed (in the split modes op(A) is split once, when it has

@@ -5,7 +5,8 @@
 //
 // Each m8n8k4 MMA is 256 fused multiply-adds in IEEE double precision, so the
 // arithmetic is the same FP64 FMA chain as the CUDA-core kernel (every element's
-// sum runs over k in ascending order, four terms per MMA); it issues one
+// sum runs over k in ascending order, four terms per MMA; where a cluster shares a
+// tile, over each CTA's part of k and then over the parts); it issues one
 // instruction where the CUDA-core kernel needs eight and reads each operand
 // element from shared memory once per warp instead of once per thread.
 //

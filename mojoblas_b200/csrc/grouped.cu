@@ -13,7 +13,7 @@
 //    tile code of gemm_f32_tile.cuh with that problem's transposes, alpha and
 //    beta (16-byte copies where that problem's operands allow them).
 //  * strsm (left side, any uplo / trans / diag, n <= 256): problems are cut
-//    into strips of 32 right-hand sides, each solved by one or two warps
+//    into strips of 32 right-hand sides, each solved by one, two or four warps
 //    (warp_solve.cuh: rows of one right-hand side in one thread's registers, the
 //    reference's column substitution, src/level3/trsm.mojo:111-168, on 32-row blocks);
 //    the plan packs the strips into CTAs of four warps, largest problems first.
@@ -292,6 +292,7 @@ int mbg_sgemm_grouped_plan(int mode, int count, const mbg_sgemm_problem* probs, 
     *out = nullptr;
     if (mode != MBG_MODE_PLAIN && mode != MBG_MODE_BF16X3 && mode != MBG_MODE_BF16X6) return MBG_ERR_INVALID_MODE;
     if (count < 0 || (count > 0 && !probs)) return MBG_ERR_INVALID_MODE;
+    DevicePointers on_device;
     for (int i = 0; i < count; ++i) {  // argument checks per problem, numbered as gemm numbers them
         const mbg_sgemm_problem& q = probs[i];
         const char ta = q.trans_a, tb = q.trans_b;
@@ -309,8 +310,7 @@ int mbg_sgemm_grouped_plan(int mode, int count, const mbg_sgemm_problem* probs, 
                           std::to_string(info));
             return info;
         }
-        if (q.m > 0 && q.n > 0 && (!is_device_pointer(q.c) ||
-                                    (q.k > 0 && (!is_device_pointer(q.a) || !is_device_pointer(q.b))))) {
+        if (q.m > 0 && q.n > 0 && (!on_device(q.c) || (q.k > 0 && (!on_device(q.a) || !on_device(q.b))))) {
             set_error_msg("grouped sgemm: problem " + std::to_string(i) + " has a host pointer (device only)");
             return MBG_ERR_UNSUPPORTED;
         }
@@ -403,6 +403,7 @@ int mbg_strsm_grouped_plan(int mode, int count, const mbg_strsm_problem* probs, 
     std::vector<TrsmDesc> v;
     v.reserve(count);
     i64 cols = 0;
+    DevicePointers on_device;
     for (int i = 0; i < count; ++i) {
         const mbg_strsm_problem& q = probs[i];
         int info = 0;  // numbered as trsm numbers them (src/level3/trsm.mojo:62-89)
@@ -419,7 +420,7 @@ int mbg_strsm_grouped_plan(int mode, int count, const mbg_strsm_problem* probs, 
                           std::to_string(info));
             return info;
         }
-        if (q.m > 0 && q.n > 0 && (!is_device_pointer(q.a) || !is_device_pointer(q.b))) {
+        if (q.m > 0 && q.n > 0 && (!on_device(q.a) || !on_device(q.b))) {
             set_error_msg("grouped strsm: problem " + std::to_string(i) + " has a host pointer (device only)");
             return MBG_ERR_UNSUPPORTED;
         }

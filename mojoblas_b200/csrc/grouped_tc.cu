@@ -461,40 +461,48 @@ grouped_tc_kernel(const TcTile* __restrict__ tiles, int ntiles, int* err) {
 // the tuning table's size class), its tiles ordered by reduction length, longest first.
 int grouped_tc_build(int terms, int count, const mbg_sgemm_problem* probs, GroupedTcPlan& out) {
     using namespace gtc;
-    std::vector<TcTile> t;
+    struct Place {  // what is sorted: the descriptors are five times as large
+        int prob, tm, tn, nkb;
+    };
+    std::vector<Place> order;
+    order.reserve(size_t(count) * 4);
     out.terms = terms;
     out.count = 0;
     for (int i = 0; i < count; ++i) {
         const mbg_sgemm_problem& q = probs[i];
         if (q.m == 0 || q.n == 0) continue;
         ++out.count;
-        const bool ta = is_t(q.trans_a), tb = is_t(q.trans_b);
-        const int bn = grouped_tc_tile_cols(q.m, q.n, q.k, ta, tb);
-        TcTile d{};
-        d.lda = q.lda; d.ldb = q.ldb; d.ldc = q.ldc;
-        const KSlabs slabs = k_slabs(q.alpha == 0.0f ? 0 : q.k, GBK);
-        if (slabs.n > 0x7fffffff) return MBG_ERR_UNSUPPORTED;  // k > 2^36: one row of op(A) takes 256 GB
-        d.nkb = int(slabs.n);
-        d.last = slabs.last;
-        d.bn = bn;
-        d.alpha = q.alpha; d.beta = q.beta;
-        for (i64 n0 = 0; n0 < q.n; n0 += bn)
-            for (i64 m0 = 0; m0 < q.m; m0 += BM) {
-                d.a = q.a + (d.nkb ? (ta ? m0 * q.lda : m0) : 0);
-                d.b = q.b + (d.nkb ? (tb ? n0 : n0 * q.ldb) : 0);
-                d.c = q.c + m0 + n0 * q.ldc;
-                d.kcontig = (ta ? 1 : 0) | (tb ? 0 : 2);
-                if (ta && q.lda % 2 == 0 && reinterpret_cast<uintptr_t>(d.a) % 8 == 0) d.kcontig |= 4;
-                if (!tb && q.ldb % 2 == 0 && reinterpret_cast<uintptr_t>(d.b) % 8 == 0) d.kcontig |= 8;
-                d.rows = int(imin(i64(BM), q.m - m0));
-                d.cols = int(imin(i64(bn), q.n - n0));
-                t.push_back(d);
-            }
+        const i64 nkb = k_slabs(q.alpha == 0.0f ? 0 : q.k, GBK).n;
+        const i64 tn = cdiv(q.n, grouped_tc_tile_cols(q.m, q.n, q.k, is_t(q.trans_a), is_t(q.trans_b))), tm = cdiv(q.m, BM);
+        // (k > 2^36: one row of op(A) takes 256 GB)
+        if (nkb > 0x7fffffff || tm > 0x3fffffff || tn > 0x3fffffff || tm * tn > 0x3fffffff) return MBG_ERR_UNSUPPORTED;
+        for (int n = 0; n < int(tn); ++n)
+            for (int m = 0; m < int(tm); ++m) order.push_back(Place{i, m, n, int(nkb)});
     }
-    if (t.size() > 0x3fffffff) return MBG_ERR_UNSUPPORTED;
-    std::stable_sort(t.begin(), t.end(), [](const TcTile& x, const TcTile& y) { return x.nkb > y.nkb; });
-    out.ntiles = int(t.size());
+    if (order.size() > 0x3fffffff) return MBG_ERR_UNSUPPORTED;
+    std::stable_sort(order.begin(), order.end(), [](const Place& x, const Place& y) { return x.nkb > y.nkb; });
+    out.ntiles = int(order.size());
     if (out.ntiles == 0) return MBG_OK;
+    std::vector<TcTile> t(order.size());
+    for (size_t i = 0; i < order.size(); ++i) {
+        const mbg_sgemm_problem& q = probs[order[i].prob];
+        const bool ta = is_t(q.trans_a), tb = is_t(q.trans_b);
+        TcTile& d = t[i];
+        d.bn = grouped_tc_tile_cols(q.m, q.n, q.k, ta, tb);
+        const i64 m0 = i64(order[i].tm) * BM, n0 = i64(order[i].tn) * d.bn;
+        d.nkb = order[i].nkb;
+        d.last = k_slabs(d.nkb ? q.k : 0, GBK).last;
+        d.lda = q.lda; d.ldb = q.ldb; d.ldc = q.ldc;
+        d.a = q.a + (d.nkb ? (ta ? m0 * q.lda : m0) : 0);
+        d.b = q.b + (d.nkb ? (tb ? n0 : n0 * q.ldb) : 0);
+        d.c = q.c + m0 + n0 * q.ldc;
+        d.kcontig = (ta ? 1 : 0) | (tb ? 0 : 2);
+        if (ta && q.lda % 2 == 0 && reinterpret_cast<uintptr_t>(d.a) % 8 == 0) d.kcontig |= 4;
+        if (!tb && q.ldb % 2 == 0 && reinterpret_cast<uintptr_t>(d.b) % 8 == 0) d.kcontig |= 8;
+        d.rows = int(imin(i64(BM), q.m - m0));
+        d.cols = int(imin(i64(d.bn), q.n - n0));
+        d.alpha = q.alpha; d.beta = q.beta;
+    }
     const size_t bytes = sizeof(TcTile) * t.size();
     MBG_CUDA(cudaMalloc(&out.table, bytes));
     MBG_CUDA(cudaMemcpy(out.table, t.data(), bytes, cudaMemcpyHostToDevice));

@@ -162,6 +162,17 @@ struct Operand {
     int finish();  // copies back if staged && copy_out
 };
 bool is_device_pointer(const void* p);
+
+// is_device_pointer for the many operands of a grouped plan, most of which lie in a few allocations: those
+// already seen are answered by their bounds, without asking the driver.  For one call's use.
+class DevicePointers {
+    struct Range { uintptr_t lo, hi; };
+    Range seen[4] = {};
+    int next = 0, asked = 0, known = 0;
+
+public:
+    bool operator()(const void* p);
+};
 bool is_pinned_host(const void* p);  // page-locked host memory (cudaHostAlloc / cudaHostRegister)
 // Host <-> device 2-D copies (width bytes x height rows, pitches in bytes; staging.cu).
 // Pageable host memory goes through page-locked bounce buffers, packed / unpacked by

@@ -2,6 +2,8 @@
 // staging, the device error flag and optional per-kernel timing.
 #include "mbg_internal.cuh"
 
+#include <cuda.h>
+
 #include <atomic>
 #include <cctype>
 #include <map>
@@ -155,6 +157,36 @@ bool is_device_pointer(const void* p) {
         return false;
     }
     return attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged;
+}
+
+bool DevicePointers::operator()(const void* p) {
+    const uintptr_t v = reinterpret_cast<uintptr_t>(p);
+    for (const Range& r : seen)
+        if (v >= r.lo && v < r.hi) {
+            ++known;
+            return true;
+        }
+    if (!is_device_pointer(p)) return false;
+    if (asked > 16 + known) return true;  // an allocation each: their bounds are not worth asking for
+    ++asked;
+    using Fn = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);
+    static const Fn fn = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<Fn>(f);
+    }();
+    CUdeviceptr base = 0;
+    size_t bytes = 0;
+    if (fn && fn(&base, &bytes, CUdeviceptr(v)) == CUDA_SUCCESS) {
+        seen[next] = Range{uintptr_t(base), uintptr_t(base) + bytes};
+        next = (next + 1) % 4;
+    }
+    return true;
 }
 
 int Operand::prepare(const void* p, i64 r, i64 c, i64 l, size_t e, bool copy_in, bool out) {
